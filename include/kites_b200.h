@@ -53,6 +53,12 @@ typedef enum kites_op {
  * AUTO lets the learned selector pick per iteration, falling back to PLAIN
  * when the predicted gain is under the margin.  The others force one
  * strategy for every iteration (used to record training timings).
+ * PLAIN runs of SSSP, BFS and CC on directed graphs with vertex_per_group 1
+ * go through one kernel that relaxes the out-edges of the changed vertices
+ * until nothing changes (same fixed point); so do AUTO runs while the
+ * selector, its margin and its coarse class are the defaults.  A host-driven
+ * loop (device_loop 0), time_kernels, record_iterations, an iteration limit
+ * or kites_graph_set_density keep the pull iteration above.
  * Batched runs (kites_sssp_batch) take PLAIN, AUTO, PUSH, PULL_ALL and
  * PULL_CHANGED; there PUSH and PULL_CHANGED move only the 32-byte sectors of
  * each source row that changed in the previous iteration, and PULL_ALL
@@ -159,7 +165,8 @@ typedef struct kites_run_stats {
   uint64_t iterations;              /* kernel iterations, as compute.cuh:135 counts */
   double device_ms;                 /* CUDA-event time of the iteration loop */
   double host_ms;                   /* wall time of the whole call           */
-  uint64_t edges_traversed;         /* sum over iterations of in-edges of active vertices */
+  uint64_t edges_traversed;         /* sum over iterations of in-edges of active vertices
+                                       (out-edges of changed ones where a run pushes) */
   uint64_t algorithmic_bytes;       /* sum over iterations of B_t            */
   uint64_t strategy_hist[KITES_STRATEGY_COUNT];
   uint64_t kernel_launches;         /* engine kernels launched by the call   */
@@ -401,7 +408,8 @@ int kites_autotune(kites_engine *eng, kites_graph *g, int op, const uint32_t *so
                    uint32_t n_sources, uint32_t batch, kites_tune_result *out);
 /* Sets the two densities by hand: the plain loop's pull uses the staged sweep
  * when the activation edges exceed dense_edges, its activation when the
- * changed rows exceed dense_rows (0 = always, UINT64_MAX = never). */
+ * changed rows exceed dense_rows (0 = always, UINT64_MAX = never).  A graph
+ * with densities set runs PLAIN and AUTO iteration by iteration. */
 int kites_graph_set_density(kites_graph *g, uint64_t dense_edges, uint64_t dense_rows);
 /* How kites_sssp_batch fetches the K-wide source rows (no counterpart in the
  * reference, whose kernels run one source at a time): 2 (default) = per-lane

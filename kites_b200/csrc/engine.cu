@@ -13,6 +13,7 @@
 #include <cub/device/device_scan.cuh>
 
 #include "engine.cuh"
+#include "frontier.cuh"
 #include "kernels.cuh"
 #include "kernels_batch.cuh"
 #include "kernels_batch_async.cuh"
@@ -77,7 +78,7 @@ int dev_alloc(kites_engine *eng, void **p, size_t bytes) {
 int run_error(uint32_t err) {
   if (err & kErrWait)
     return fail(KITES_ERR_TIMEOUT,
-                "a bounded wait on a TMA row copy gave up (error bits 0x%x)", err);
+                "a bounded wait inside a kernel gave up (error bits 0x%x)", err);
   return fail(KITES_ERR_CUDA,
               "a kernel read an out-of-range vertex or edge index and skipped it "
               "(error bits 0x%x)", err);
@@ -744,6 +745,69 @@ int run_pagerank(kites_graph *g, uint64_t n_real, float *out, const kites_run_op
                       std::chrono::steady_clock::now() - t0).count();
   }
   return KITES_OK;
+}
+
+// ---- the single-launch frontier loop -------------------------------------------
+
+// Whether a run goes through k_frontier_run: a vertex-level directed graph
+// and a program whose comp(INF) is INF, and a caller that asks for nothing
+// that only the iteration-by-iteration loop has (host-driven iterations,
+// per-iteration times or records, an iteration limit, densities set by hand).
+// AUTO takes it while the selector's weights, margin and coarse class are the
+// defaults: against the selector's mix it ran R-MAT of 2.0 M vertices and 32 M
+// edges in 0.95 against 1.41 ms (SSSP) and an Erdos-Renyi graph of 2^20
+// vertices and 2^24 edges in 0.26 against 0.56 ms (BFS); weights loaded or
+// trained by the caller make per-iteration picks.
+bool frontier_applies(const kites_graph *g, int op, const kites_run_opts &o) {
+  if (g->vpg != 1 || !g->directed || g->vsize != 4 || !g->outR || !g->outE) return false;
+  if (op != OP_SSSP && op != OP_BFS && op != OP_CC) return false;
+  if (op == OP_SSSP && g->esize != 4) return false;
+  if (!o.device_loop || o.time_kernels || o.record_iterations || o.max_iterations) return false;
+  if (g->density_set || g->tuning || g->n + g->m / kSeg > 0xFFF00000ull) return false;
+  if (o.strategy == KITES_STRATEGY_PLAIN) return true;
+  return o.strategy == KITES_STRATEGY_AUTO && g->eng->sel_default && o.selector_margin < 0.f &&
+         g->coarse_strategy == KITES_STRATEGY_PULL_ALL;
+}
+
+// Runs `op` from the start `seed` describes.  KITES_ERR_UNSUPPORTED (without
+// a message) when the caller's state (kSeedFinite) is not one the loop may
+// start from: nothing has been changed then.
+int run_frontier(kites_graph *g, int op, int seed, uint32_t source, kites_run_stats *st) {
+  auto t0 = std::chrono::steady_clock::now();
+  frontier_result r;
+  float ms = 0.f;
+  KITES_TRY(launch_frontier(g, op, seed, source, &r, &ms));
+  if (r.error) return run_error(r.error);
+  if (r.violated) return KITES_ERR_UNSUPPORTED;
+  if (st) {
+    memset(st, 0, sizeof(*st));
+    st->iterations = std::max<unsigned long long>(r.iterations, 1);
+    st->device_ms = ms;
+    st->edges_traversed = r.relaxed;
+    // Per queued vertex its offsets and value, per out-edge C + eT + V, per
+    // lowered value its store and queue entry.
+    const uint64_t e_bytes = op == OP_SSSP ? 4 : 0;
+    st->algorithmic_bytes = 20ull * r.active + (8ull + e_bytes) * r.relaxed + 12ull * r.updated;
+    st->strategy_hist[KITES_STRATEGY_PLAIN] = st->iterations;
+    st->kernel_launches = 1;
+    st->host_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
+  }
+  return KITES_OK;
+}
+
+// Whether this call runs as the frontier loop, with its buffers in place.  A
+// graph whose queues do not fit in memory goes to the per-iteration loop.
+bool frontier_ready(kites_graph *g, int op, const kites_run_opts *opts) {
+  kites_run_opts o;
+  kites_default_run_opts(&o);
+  if (opts) o = *opts;
+  if (!frontier_applies(g, op, o)) return false;
+  if (g->fr_mem) return true;
+  size_t queues;
+  if (graph_alloc(g, &g->fr_mem, frontier_bytes(g, &queues)) == KITES_OK) return true;
+  g->fr_mem = nullptr;
+  clear_error();
+  return false;
 }
 
 // ---- flexible loop: one strategy per iteration -------------------------------
@@ -2534,10 +2598,9 @@ extern "C" int kites_graph_set_frontier(kites_graph *g, const uint32_t *bits, ui
   return KITES_OK;
 }
 
-extern "C" int kites_process(kites_engine *eng, kites_graph *g, int op,
-                             const kites_run_opts *opts, kites_run_stats *stats) {
-  clear_error();
-  KITES_TRY(check_graph(eng, g));
+// The plain per-iteration loop from the graph's values and frontier.
+static int run_plain_op(kites_graph *g, int op, const kites_run_opts *opts,
+                        kites_run_stats *stats) {
   if (op < 0 || op > OP_PR) return fail(KITES_ERR_INVALID, "unknown operator %d", op);
   if (op == OP_PR) return fail(KITES_ERR_UNSUPPORTED, "use kites_pagerank");
   if (g->vsize != 4) return fail(KITES_ERR_UNSUPPORTED, "built-in operators need 4-byte vertex values");
@@ -2549,6 +2612,17 @@ extern "C" int kites_process(kites_engine *eng, kites_graph *g, int op,
     return fail(KITES_ERR_UNSUPPORTED, "strategy %d not available for kites_process", o.strategy);
   return g->off64 ? dispatch_process<uint64_t>(g, op, o, stats)
                   : dispatch_process<uint32_t>(g, op, o, stats);
+}
+
+extern "C" int kites_process(kites_engine *eng, kites_graph *g, int op,
+                             const kites_run_opts *opts, kites_run_stats *stats) {
+  clear_error();
+  KITES_TRY(check_graph(eng, g));
+  if ((!opts || opts->strategy == KITES_STRATEGY_PLAIN) && frontier_ready(g, op, opts)) {
+    const int st = run_frontier(g, op, kSeedFinite, 0, stats);
+    if (st != KITES_ERR_UNSUPPORTED) return st;
+  }
+  return run_plain_op(g, op, opts, stats);
 }
 
 // Runs `op` with a strategy other than PLAIN from the changed set already in
@@ -2572,6 +2646,21 @@ static int run_strategies(kites_engine *eng, kites_graph *g, int op, const kites
                   : dispatch_flex<uint32_t>(g, op, o, stats);
 }
 
+// Ends a single-source style call: the values to dist_out (host or device
+// memory, may be null) and the call's wall time since t0.
+static int copy_values(kites_graph *g, uint32_t *dist_out, kites_run_stats *stats,
+                       std::chrono::steady_clock::time_point t0) {
+  cudaStream_t s = g->eng->stream;
+  if (dist_out) {
+    KITES_CUDA_TRY(cudaMemcpyAsync(dist_out, g->V, g->n_given * 4, cudaMemcpyDefault, s));
+    KITES_CUDA_TRY(cudaStreamSynchronize(s));
+  }
+  if (stats)
+    stats->host_ms = std::chrono::duration<double, std::milli>(
+                         std::chrono::steady_clock::now() - t0).count();
+  return KITES_OK;
+}
+
 extern "C" int kites_sssp(kites_engine *eng, kites_graph *g, int op, uint32_t source,
                           uint32_t *dist_out, const kites_run_opts *opts,
                           kites_run_stats *stats) {
@@ -2583,6 +2672,10 @@ extern "C" int kites_sssp(kites_engine *eng, kites_graph *g, int op, uint32_t so
   if (!g->outR) return fail(KITES_ERR_UNSUPPORTED, "graph has no out-CSR");
   cudaStream_t s = eng->stream;
   auto t0 = std::chrono::steady_clock::now();
+  if (frontier_ready(g, op, opts)) {
+    KITES_TRY(run_frontier(g, op, kSeedSource, source, stats));
+    return copy_values(g, dist_out, stats, t0);
+  }
   k_fill_u32<<<grid_for(g->n), 256, 0, s>>>((uint32_t *)g->V, g->n, kInf);
   KITES_CUDA_TRY(cudaMemsetAsync(g->bitmaps, 0, 4 * g->nwords * 4, s));
   if (opts && opts->strategy != KITES_STRATEGY_PLAIN) {
@@ -2591,14 +2684,7 @@ extern "C" int kites_sssp(kites_engine *eng, kites_graph *g, int op, uint32_t so
     KITES_CUDA_TRY(cudaGetLastError());
     int st = run_strategies(eng, g, op, opts, stats);
     if (st != KITES_OK) return st;
-    if (dist_out) {
-      KITES_CUDA_TRY(cudaMemcpyAsync(dist_out, g->V, g->n_given * 4, cudaMemcpyDefault, s));
-      KITES_CUDA_TRY(cudaStreamSynchronize(s));
-    }
-    if (stats)
-      stats->host_ms = std::chrono::duration<double, std::milli>(
-                           std::chrono::steady_clock::now() - t0).count();
-    return KITES_OK;
+    return copy_values(g, dist_out, stats, t0);
   }
   if (g->off64)
     k_seed_source<uint64_t><<<32, 256, 0, s>>>((uint32_t *)g->V, (const uint64_t *)g->outR,
@@ -2607,18 +2693,10 @@ extern "C" int kites_sssp(kites_engine *eng, kites_graph *g, int op, uint32_t so
     k_seed_source<uint32_t><<<32, 256, 0, s>>>((uint32_t *)g->V, (const uint32_t *)g->outR,
                                                g->outC, source, g->shift, g->frontier[0]);
   KITES_CUDA_TRY(cudaGetLastError());
-  int st = kites_process(eng, g, op, opts, stats);
+  int st = run_plain_op(g, op, opts, stats);
   if (st != KITES_OK) return st;
-  if (dist_out) {
-    KITES_CUDA_TRY(cudaMemcpyAsync(dist_out, g->V, g->n_given * 4, cudaMemcpyDefault, s));
-    KITES_CUDA_TRY(cudaStreamSynchronize(s));
-  }
-  if (stats) {
-    stats->kernel_launches += 2;
-    stats->host_ms = std::chrono::duration<double, std::milli>(
-                         std::chrono::steady_clock::now() - t0).count();
-  }
-  return KITES_OK;
+  if (stats) stats->kernel_launches += 2;
+  return copy_values(g, dist_out, stats, t0);
 }
 
 extern "C" int kites_cc(kites_engine *eng, kites_graph *g, uint32_t *labels_out,
@@ -2627,6 +2705,10 @@ extern "C" int kites_cc(kites_engine *eng, kites_graph *g, uint32_t *labels_out,
   KITES_TRY(check_graph(eng, g));
   cudaStream_t s = eng->stream;
   auto t0 = std::chrono::steady_clock::now();
+  if (frontier_ready(g, OP_CC, opts)) {
+    KITES_TRY(run_frontier(g, OP_CC, kSeedLabels, 0, stats));
+    return copy_values(g, labels_out, stats, t0);
+  }
   k_iota_u32<<<grid_for(g->n), 256, 0, s>>>((uint32_t *)g->V, g->n);
   KITES_CUDA_TRY(cudaMemsetAsync(g->bitmaps, 0, 4 * g->nwords * 4, s));
   const bool strategies = opts && opts->strategy != KITES_STRATEGY_PLAIN;
@@ -2636,18 +2718,10 @@ extern "C" int kites_cc(kites_engine *eng, kites_graph *g, uint32_t *labels_out,
                                                    strategies ? g->n_given : g->nbits, g->nwords);
   KITES_CUDA_TRY(cudaGetLastError());
   int st = strategies ? run_strategies(eng, g, OP_CC, opts, stats)
-                      : kites_process(eng, g, OP_CC, opts, stats);
+                      : run_plain_op(g, OP_CC, opts, stats);
   if (st != KITES_OK) return st;
-  if (labels_out) {
-    KITES_CUDA_TRY(cudaMemcpyAsync(labels_out, g->V, g->n_given * 4, cudaMemcpyDefault, s));
-    KITES_CUDA_TRY(cudaStreamSynchronize(s));
-  }
-  if (stats) {
-    stats->kernel_launches += 2;
-    stats->host_ms = std::chrono::duration<double, std::milli>(
-                         std::chrono::steady_clock::now() - t0).count();
-  }
-  return KITES_OK;
+  if (stats) stats->kernel_launches += 2;
+  return copy_values(g, labels_out, stats, t0);
 }
 
 extern "C" int kites_pagerank(kites_engine *eng, kites_graph *g, uint64_t n_real,
@@ -2737,7 +2811,10 @@ extern "C" int kites_sssp_multi_seed(kites_engine *eng, kites_graph *g, int op,
   KITES_CUDA_TRY(cudaMemcpyAsync(dseeds, hs.data(), n_seeds * 4, cudaMemcpyHostToDevice, s));
   k_fill_u32<<<grid_for(g->n), 256, 0, s>>>((uint32_t *)g->V, g->n, kInf);
   KITES_CUDA_TRY(cudaMemsetAsync(g->bitmaps, 0, 4 * g->nwords * 4, s));
-  const bool strategies = opts && opts->strategy != KITES_STRATEGY_PLAIN;
+  const bool fr = frontier_ready(g, op, opts);
+  // The frontier loop starts, as the strategy loops do, from the seeds
+  // themselves (it finds them by their value).
+  const bool strategies = fr || (opts && opts->strategy != KITES_STRATEGY_PLAIN);
   const unsigned blocks = (unsigned)std::min<uint64_t>(n_seeds, 65535);
   if (g->off64)
     k_seed_many<uint64_t><<<blocks, 128, 0, s>>>((uint32_t *)g->V, dseeds, n_seeds,
@@ -2751,17 +2828,12 @@ extern "C" int kites_sssp_multi_seed(kites_engine *eng, kites_graph *g, int op,
                                                  strategies ? 1 : 0);
   KITES_CUDA_TRY(cudaGetLastError());
   KITES_CUDA_TRY(cudaFreeAsync(dseeds, s));
-  int st = strategies ? run_strategies(eng, g, op, opts, stats)
-                      : kites_process(eng, g, op, opts, stats);
+  int st = fr ? run_frontier(g, op, kSeedZeros, 0, stats)
+              : strategies ? run_strategies(eng, g, op, opts, stats)
+                           : run_plain_op(g, op, opts, stats);
   if (st != KITES_OK) return st;
-  if (dist_out) {
-    KITES_CUDA_TRY(cudaMemcpyAsync(dist_out, g->V, g->n_given * 4, cudaMemcpyDefault, s));
-    KITES_CUDA_TRY(cudaStreamSynchronize(s));
-  }
-  if (stats)
-    stats->host_ms = std::chrono::duration<double, std::milli>(
-                         std::chrono::steady_clock::now() - t0).count();
-  return KITES_OK;
+  if (fr && stats) stats->kernel_launches += 2;
+  return copy_values(g, dist_out, stats, t0);
 }
 
 // ---- learned selector ------------------------------------------------------------
@@ -2840,8 +2912,10 @@ static int fit_selector(kites_engine *eng, const float *features, const float *t
     k_mlp_adam<<<(kParams + 255) / 256, 256, 0, s>>>(P, G, M, Vv, lr, 0.9f, 0.999f, 1e-8f, (int)e);
   }
   KITES_CUDA_TRY(cudaGetLastError());
-  if (load)
+  if (load) {
+    eng->sel_default = false;
     KITES_CUDA_TRY(cudaMemcpyAsync(eng->sel_params, P, kParams * 4, cudaMemcpyDeviceToDevice, s));
+  }
   float hloss = 0.f;
   KITES_CUDA_TRY(cudaMemcpyAsync(&hloss, loss, 4, cudaMemcpyDeviceToHost, s));
   if (params_out) KITES_CUDA_TRY(cudaMemcpyAsync(params_out, P, kParams * 4, cudaMemcpyDefault, s));
@@ -2909,6 +2983,7 @@ extern "C" int kites_selector_load(kites_engine *eng, const float *params, uint3
   if (n_params != (uint32_t)kParams)
     return fail(KITES_ERR_INVALID, "selector has %d parameters, got %u", kParams, n_params);
   KITES_TRY(set_device(eng));
+  eng->sel_default = false;
   KITES_CUDA_TRY(cudaMemcpyAsync(eng->sel_params, params, kParams * 4, cudaMemcpyDefault,
                                  eng->stream));
   KITES_CUDA_TRY(cudaStreamSynchronize(eng->stream));
@@ -2975,6 +3050,12 @@ extern "C" int kites_autotune(kites_engine *eng, kites_graph *g, int op, const u
   kites_run_opts o;
   kites_default_run_opts(&o);
   kites_run_stats st;
+  // What is tuned here belongs to the per-iteration loops, so they are timed.
+  struct tuning_scope {
+    kites_graph *g;
+    explicit tuning_scope(kites_graph *graph) : g(graph) { g->tuning = true; }
+    ~tuning_scope() { g->tuning = false; }
+  } scope(g);
   // Runs each source once (the first run of a shape also warms its loop).
   auto time_single = [&](int strategy, float *ms) -> int {
     o.strategy = strategy;
@@ -3168,6 +3249,7 @@ extern "C" int kites_graph_set_density(kites_graph *g, uint64_t dense_edges,
   KITES_CUDA_TRY(cudaStreamSynchronize(g->eng->stream));
   g->dense_edges = dense_edges;
   g->dense_rows = dense_rows;
+  g->density_set = true;
   drop_all_loops(g);  // captured loops hold the old thresholds
   return KITES_OK;
 }

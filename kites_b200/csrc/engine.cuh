@@ -24,6 +24,7 @@ struct kites_engine {
   int l2_bytes = 0;
   void *pinned = nullptr;         // small pinned scratch for flag read-backs
   float *sel_params = nullptr;    // learned selector weights (device), or null
+  bool sel_default = true;        // they are the compiled-in ones
   float *sel_params_batch = nullptr;  // the batched loop's selector weights
   std::vector<struct kites_graph *> graphs;   // live graphs, destroyed with the engine
 };
@@ -132,6 +133,10 @@ struct kites_graph {
 
   // PageRank scratch (allocated on first use).
   float *pr_x = nullptr, *pr_y = nullptr, *pr_inv_out = nullptr;
+
+  void *fr_mem = nullptr;            // k_frontier_run's buffers (allocated on first use)
+  bool density_set = false;          // kites_graph_set_density was called
+  bool tuning = false;               // kites_autotune is timing the per-iteration loops
 
   // time_kernels: one record per iteration of the last host-loop run (pull
   // time, whether the dense sweep did the pull, the counters after it).

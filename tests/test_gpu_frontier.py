@@ -1,0 +1,131 @@
+"""The single-launch frontier loop (default options of kites_sssp, kites_cc,
+kites_sssp_multi_seed and kites_process): the oracle's fixed point at the
+sizes where its queues and thresholds change shape, and the per-iteration
+loop's result from any state kites_process is given."""
+import numpy as np
+import pytest
+
+from kites_b200 import capi
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+INF = O.INF32
+OPS = [(capi.OP_SSSP, O.OP_SSSP_SAT), (capi.OP_BFS, O.OP_BFS_SAT)]
+
+
+def oracle(R, C, E, n, sources, oop):
+    V0 = np.full(n, INF, np.uint32)
+    V0[sources] = 0
+    return O.sanity_check(R, C, E, V0, op=oop)[0]
+
+
+@pytest.mark.parametrize("offsets64", [False, True])
+@pytest.mark.parametrize("deg", [1, 31, 33, 255, 256, 257, 512, 513, 4097])
+def test_row_lengths(engine, deg, offsets64):
+    """Out-rows around the lane, segment and batch sizes: two hubs of `deg`
+    out-edges in a ring that reaches every vertex."""
+    n = 5000
+    rng = np.random.default_rng(deg)
+    ring = np.arange(n, dtype=np.uint32)
+    hub = np.concatenate([rng.choice(n, deg, replace=False) for _ in range(2)]).astype(np.uint32)
+    s = np.concatenate([ring, np.repeat(np.uint32([3, 1700]), deg)]).astype(np.uint32)
+    d = np.concatenate([(ring + 1) % n, hub]).astype(np.uint32)
+    w = rng.integers(1, 200, s.shape[0], dtype=np.uint32)
+    R, C, E = capi.csc_from_edges(n, s, d, w)
+    g = capi.Graph(engine, R, C, E, offsets64=offsets64)
+    try:
+        for op, oop in OPS:
+            for src in (0, 3):
+                np.testing.assert_array_equal(g.sssp(src, op=op)[0],
+                                              oracle(R, C, E, n, [src], oop))
+        seeds = np.array([7, 1700, 4999], np.uint32)
+        np.testing.assert_array_equal(g.sssp_multi_seed(seeds)[0],
+                                      oracle(R, C, E, n, seeds, O.OP_SSSP_SAT))
+        np.testing.assert_array_equal(g.cc()[0], np.zeros(n, np.uint32))
+    finally:
+        g.close()
+
+
+@pytest.mark.parametrize("w_hi", [1, 7, 1000, 2**31, 2**32 - 1])
+@pytest.mark.parametrize("kind", ["grid", "sparse"])
+def test_thresholds(engine, kind, w_hi):
+    """Graphs with few edges a vertex order their work by a threshold: unit
+    weights, small and large ones, and ones whose sums saturate."""
+    rng = np.random.default_rng(w_hi % 1000)
+    if kind == "grid":
+        n = 70 * 70
+        s, d, _ = capi.gen_grid(70, seed=3)
+    else:
+        n = 20001
+        s = rng.integers(0, n, 3 * n, dtype=np.uint32)
+        d = rng.integers(0, n, 3 * n, dtype=np.uint32)
+    w = rng.integers(1, w_hi, s.shape[0], dtype=np.uint64, endpoint=True).astype(np.uint32)
+    R, C, E = capi.csc_from_edges(n, s, d, w)
+    g = capi.Graph(engine, R, C, E)
+    try:
+        for src in (0, n // 2):
+            np.testing.assert_array_equal(g.sssp(src)[0],
+                                          oracle(R, C, E, n, [src], O.OP_SSSP_SAT))
+    finally:
+        g.close()
+
+
+@pytest.mark.parametrize("scale,factor", [(15, 16), (18, 16), (20, 17)])
+def test_wide_iterations(engine, scale, factor):
+    """Iterations above the short size, and (from 16 M edges) a threshold on
+    an R-MAT graph: the values of the per-iteration loop, whose first
+    iteration from them changes nothing."""
+    n = 1 << scale
+    s, d, w = capi.gen_rmat(scale, factor * n, seed=scale)
+    g = capi.Graph.from_edges(engine, n, s, d, w)
+    try:
+        src = int(s[12345])
+        loop = capi.default_opts(device_loop=0)
+        for op, _ in OPS:
+            dist, _ = g.sssp(src, op=op)
+            np.testing.assert_array_equal(dist, g.sssp(src, op=op, opts=loop)[0])
+        np.testing.assert_array_equal(g.cc()[0], g.cc(opts=loop)[0])
+    finally:
+        g.close()
+
+
+@pytest.mark.parametrize("op,oop", OPS + [(capi.OP_CC, None)])
+@pytest.mark.parametrize("state", ["sources", "missing", "partial", "empty", "settled"])
+def test_process_states(engine, op, oop, state):
+    """kites_process from a caller's values and frontier gives what the
+    per-iteration loop gives, also where an unsatisfied edge leads outside
+    the frontier, and leaves an empty frontier."""
+    n = 3001
+    s, d, w = capi.gen_rmat(12, 20000, seed=5, n_vertices=n)
+    R, C, E = capi.csc_from_edges(n, s, d, w)
+    rng = np.random.default_rng(11)
+    V = np.full(n, INF, np.uint32)
+    bits = np.zeros(n, bool)
+    srcs = s[[5, 500, 5000]]
+    V[srcs] = [0, 40, 7]
+    if state == "sources":
+        bits[d[np.isin(s, srcs)]] = True
+    elif state == "missing":         # one source's out-neighbours are not in the frontier
+        bits[d[np.isin(s, srcs[:2])]] = True
+    elif state == "partial":
+        V = rng.integers(0, 500, n, dtype=np.uint32)
+        bits = rng.random(n) < 0.3
+    elif state == "settled":
+        V[:] = 0
+        bits[:] = True
+    words = np.packbits(np.pad(bits, (0, -n % 32)), bitorder="little").view(np.uint32)
+    got = []
+    g = capi.Graph(engine, R, C, E)
+    try:
+        for loop in (1, 0):
+            g.set_values(V)
+            g.set_frontier(words, n)
+            st = g.process(op, opts=capi.default_opts(device_loop=loop))
+            assert st.iterations >= 1
+            got.append(g.get_values(n))
+            g.process(op, opts=capi.default_opts(device_loop=loop))
+            np.testing.assert_array_equal(g.get_values(n), got[-1])
+        np.testing.assert_array_equal(got[0], got[1])
+    finally:
+        g.close()
