@@ -709,22 +709,47 @@ int run_pagerank(kites_graph *g, uint64_t n_real, float *out, const kites_run_op
   auto t0 = std::chrono::steady_clock::now();
   void *p;
   if (!g->pr_x) {
-    KITES_TRY(graph_alloc(g, &p, g->n * 4)); g->pr_x = (float *)p;
-    KITES_TRY(graph_alloc(g, &p, g->n * 4)); g->pr_y = (float *)p;
-    KITES_TRY(graph_alloc(g, &p, g->n * 4)); g->pr_inv_out = (float *)p;
+    // x of this step and the next, the split rows' sums, 1 / out-degree.
+    KITES_TRY(graph_alloc(g, &p, 4 * g->n * 4));
+    g->pr_x = (float *)p;
   }
-  float *pr = (float *)g->V;
-  k_pr_init<<<grid_for(g->n), 256, 0, s>>>(g->out_deg, g->n, n_real, g->pr_inv_out,
-                                           g->pr_x, g->pr_y, pr);
+  if (!g->rowid && !g->pr_rowid && g->m) {   // vertex groups have no sweeps' row index
+    KITES_TRY(graph_alloc(g, &p, g->m * 4));
+    g->pr_rowid = (uint32_t *)p;
+    k_row_of_edge<OffT><<<grid_for(g->m), 256, 0, s>>>((const OffT *)g->R, g->n + 1, g->m,
+                                                      g->pr_rowid);
+  }
+  float *x[2] = {g->pr_x, g->pr_x + g->n};
+  float *pr = (float *)g->V, *inv_out = g->pr_x + 3 * g->n;
+  pr_args<OffT> a{};
+  a.R = (const OffT *)g->R;
+  a.C = g->C;
+  a.rowid = g->rowid ? g->rowid : g->pr_rowid;
+  a.m = g->m;
+  a.n_real = n_real;
+  a.y = g->pr_x + 2 * g->n;
+  a.inv_out = inv_out;
+  a.base = (float)((1.0 - (double)o.damping) / (double)n_real);
+  a.damping = o.damping;
+  int per_sm = 0;
+  KITES_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pr_pull<OffT>,
+                                                               kSweepThreads, 0));
+  const uint64_t chunks = (g->m + kPrChunk - 1) / kPrChunk;
+  const unsigned grid = grid_for(chunks * 32, kSweepThreads,
+                                 (unsigned)(std::max(per_sm, 1) * eng->sm_count));
+  k_pr_init<OffT><<<grid_for(g->n), 256, 0, s>>>(a, g->out_deg, g->n, o.pagerank_iterations,
+                                                 inv_out, x[0], x[1], pr);
   KITES_CUDA_TRY(cudaGetLastError());
-  chunk_geom<OffT> gin{(const OffT *)g->R, g->C, g->chunk_in, g->nchunks_in,
-                       g->n, g->n + g->m, g->chunk_items};
-  const float base = (float)((1.0 - (double)o.damping) / (double)n_real);
+  uint64_t launches = 1;
   KITES_CUDA_TRY(cudaEventRecord(eng->ev0, s));
-  for (uint32_t it = 0; it < o.pagerank_iterations; ++it) {
-    k_pr_pull<OffT><<<g->pull_grid, kBlock, 0, s>>>(gin, g->pr_x, g->pr_y);
-    k_pr_update<<<grid_for(n_real), 256, 0, s>>>(n_real, base, o.damping, g->pr_inv_out,
-                                                 g->pr_x, g->pr_y, pr);
+  for (uint32_t it = 0; it < o.pagerank_iterations && g->m; ++it) {
+    a.x = x[it & 1];
+    a.x_next = x[(it & 1) ^ 1];
+    a.pr = it + 1 == o.pagerank_iterations ? pr : nullptr;
+    k_pr_pull<OffT><<<grid, kSweepThreads, 0, s>>>(a);
+    if (chunks > 1) k_pr_join<OffT><<<grid_for(chunks - 1), 256, 0, s>>>(a);
+    if (it == 0) k_pr_empty<OffT><<<grid_for(n_real), 256, 0, s>>>(a, x[0]);
+    launches += (chunks > 1 ? 2 : 1) + (it == 0 ? 1 : 0);
   }
   KITES_CUDA_TRY(cudaGetLastError());
   KITES_CUDA_TRY(cudaEventRecord(eng->ev1, s));
@@ -736,11 +761,10 @@ int run_pagerank(kites_graph *g, uint64_t n_real, float *out, const kites_run_op
     st->iterations = o.pagerank_iterations;
     st->device_ms = ms;
     st->edges_traversed = (uint64_t)o.pagerank_iterations * g->m;
-    // Per step: C and the x[u] gather per edge, R per row, then y/inv/x/pr.
-    st->algorithmic_bytes = (uint64_t)o.pagerank_iterations *
-                            (8ull * g->m + (g->off64 ? 8ull : 4ull) * g->n + 20ull * n_real);
+    // Per step: C, the row index and the x[u] gather per edge, inv and x per row.
+    st->algorithmic_bytes = (uint64_t)o.pagerank_iterations * (12ull * g->m + 8ull * n_real);
     st->strategy_hist[KITES_STRATEGY_PULL_ALL] = o.pagerank_iterations;
-    st->kernel_launches = 1 + 2ull * o.pagerank_iterations;
+    st->kernel_launches = launches;
     st->host_ms = std::chrono::duration<double, std::milli>(
                       std::chrono::steady_clock::now() - t0).count();
   }

@@ -132,7 +132,8 @@ struct kites_graph {
   float auto_margin_batch = -1.f;    // the same for the batched AUTO loops
 
   // PageRank scratch (allocated on first use).
-  float *pr_x = nullptr, *pr_y = nullptr, *pr_inv_out = nullptr;
+  float *pr_x = nullptr;         // x twice, split rows' sums, 1 / out-degree: n each
+  uint32_t *pr_rowid = nullptr;  // row of every in-edge where there is no rowid
 
   void *fr_mem = nullptr;            // k_frontier_run's buffers (allocated on first use)
   bool density_set = false;          // kites_graph_set_density was called
