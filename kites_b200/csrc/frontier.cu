@@ -26,6 +26,8 @@ int launch(kites_graph *g, int seed, uint32_t source, frontier_result *out, floa
   frontier_args<OffT> a{};
   a.outR = (const OffT *)g->outR;
   a.outC = g->outC;
+  a.R = (const OffT *)g->R;
+  a.C = g->C;
   a.outE = g->outE;
   a.out_deg = g->out_deg;
   a.V = (uint32_t *)g->V;

@@ -39,8 +39,8 @@
 // 7,115 vertices and 103,689 edges 501 -> 199 us (kites_process, values to and
 // from the host); R-MAT 2^22 vertices, 2^26 edges SSSP 2.49 -> 1.01 ms (4.22
 // with another source); grid 512 x 512 22.9 -> 5.9 ms; BFS on 60,013 vertices
-// and 983,040 edges 379 -> 114 us; min labels of a symmetrised R-MAT of 2^20
-// vertices and 2^25 edges 720 -> 452 us; 64 R-MAT graphs in one run (768,000
+// and 983,040 edges 379 -> 109 us; min labels of a symmetrised R-MAT of 2^20
+// vertices and 2^25 edges 720 -> 281 us; 64 R-MAT graphs in one run (768,000
 // vertices, 12.3 M edges) 1.61 -> 0.72 ms.
 #pragma once
 #include "common.cuh"
@@ -89,7 +89,8 @@ struct frontier_ctl {
 
 template <typename OffT>
 struct frontier_args {
-  const OffT *outR;
+  const OffT *R, *outR;   // in- and out-rows
+  const uint32_t *C;
   const uint32_t *outC, *outE, *out_deg;
   uint32_t *V;
   uint64_t n, m;
@@ -185,10 +186,14 @@ struct frontier_run {
   // they are); the far ones to list buf, counted in far_n[cnt].
   __device__ void flush(uint32_t near, uint32_t far, uint32_t buf, uint32_t cnt) {
     __syncwarp();
-    uint32_t base = 0;
-    if (lane == 0 && near) base = atomicAdd(&next()->qn, near);
-    if (lane == 1 && far) base = atomicAdd(&a.ctl->far_n[cnt], far);
-    const uint32_t qb = __shfl_sync(kFull, base, 0), fb = __shfl_sync(kFull, base, 1);
+    // Both counters' round trips at once.
+    uint32_t qb = 0, fb = 0;
+    if (lane == 0) {
+      if (near) qb = atomicAdd(&next()->qn, near);
+      if (far) fb = atomicAdd(&a.ctl->far_n[cnt], far);
+    }
+    qb = __shfl_sync(kFull, qb, 0);
+    fb = __shfl_sync(kFull, fb, 0);
     n_near -= near;
     n_far -= far;
     for (uint32_t i = lane; i < near; i += 32) a.q[qp ^ 1u][qb + i] = sm.near[wib][n_near + i];
@@ -298,7 +303,7 @@ struct frontier_run {
       for (int k = 0; k < kPer; ++k) {
         const uint32_t i = lane + 32 * k;
         nd[k] = kInf;
-        old[k] = 0;
+        old[k] = deg[k] = 0;
         v[k] = 0;
         if (i < take) {
           const uint2 c = sm.cand[wib][n_cand + i];
@@ -319,11 +324,14 @@ struct frontier_run {
           n_updated += 1;
           const uint32_t bit = 1u << (v[k] & 31u);
           uint32_t *set = near[k] ? queued(qp ^ 1u) : far_bits();
+          // (a short iteration looks without waiting for the bit)
+          if (kPer <= kShortCand) deg[k] = near[k] ? a.out_deg[v[k]] : 0u;
           if (atomicOr(set + (v[k] >> 5), bit) & bit) near[k] = far[k] = false;
         }
       }
 #pragma unroll
-      for (int k = 0; k < kPer; ++k) deg[k] = near[k] ? a.out_deg[v[k]] : 0u;
+      for (int k = 0; k < kPer; ++k)
+        if (kPer > kShortCand) deg[k] = near[k] ? a.out_deg[v[k]] : 0u;
 #pragma unroll
       for (int k = 0; k < kPer; ++k)
         if (__any_sync(kFull, near[k] || far[k]))
@@ -422,13 +430,15 @@ struct frontier_run {
   // log2 of the whole rows that hold about `edges` out-edges, at most a lane
   // each.
   __device__ uint32_t rows_of(const frontier_slot &sl, uint32_t edges) const {
-    uint32_t log = 0;
-    while (log < 5u && (2ull << log) * sl.row_edges <= (unsigned long long)edges * sl.qn) ++log;
-    return log;
+    const float rows = (float)edges * (float)sl.qn / fmaxf((float)sl.row_edges, 1.f);
+    return 31u - __clz((uint32_t)fminf(fmaxf(rows, 1.f), 32.f));
   }
 
   // A short iteration: every warp takes at most a segment or some rows with
-  // two windows of out-edges, all at once.
+  // two windows of out-edges, all at once.  (Letting a warp go on with the
+  // vertices it queued itself before the grid meets relaxed so much out of
+  // order that R-MAT of 7,115 vertices took 323 us against 208 and the 512 x
+  // 512 grid gained nothing.)
   __device__ void short_push(const frontier_slot &sl) {
     const uint32_t log = rows_of(sl, 64 * kShortFlight);
     const uint32_t rows = 1u << log, jobs = sl.bn + ((sl.qn + rows - 1u) >> log);
@@ -559,7 +569,13 @@ struct frontier_run {
       if (blockIdx.x == 0 && wib == 0)
         push(lane == 0, false, a.source, a.out_deg[a.source], fc, far_c);
     } else if (a.seed == kSeedLabels) {
-      for (uint64_t v = t0; v < a.n; v += stride) a.V[v] = (uint32_t)v;
+      // Any in-neighbour's id is a label that reaches v; rows are sorted as a
+      // rule, so the first is the least.
+      for (uint64_t v = t0; v < a.n; v += stride) {
+        const OffT r = a.R[v];
+        const uint32_t id = (uint32_t)v;
+        a.V[v] = r < a.R[v + 1] ? min(id, a.C[r]) : id;
+      }
     }
     for (uint64_t w = t0; w < 3 * a.nwords; w += stride) a.bits[w] = 0u;
     if (a.seed != kSeedFinite)
@@ -630,7 +646,15 @@ struct frontier_run {
     } else if (a.seed == kSeedFinite) {
       seed_all([&](uint32_t v) { return __ldcg(a.V + v) != kInf; });
     } else if (a.seed == kSeedLabels) {
-      seed_all([](uint32_t) { return true; });
+      // The label of a vertex's label reaches it too (whichever values the
+      // others have got by now).  On R-MAT most labels are final after this,
+      // and the iteration over every edge lowers few: 467 -> 281 us for the
+      // symmetrised graph of 2^20 vertices and 2^25 edges.
+      seed_all([&](uint32_t v) {
+        const uint32_t l = __ldcg(a.V + v), ll = __ldcg(a.V + l);
+        if (ll < l) atomicMin(a.V + v, ll);
+        return true;
+      });
     }
     if (a.seed != kSeedSource && !end(fc, far_c)) return finish(false, true);
     qp ^= 1u;
