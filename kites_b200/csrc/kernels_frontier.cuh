@@ -39,7 +39,7 @@
 // 7,115 vertices and 103,689 edges 501 -> 199 us (kites_process, values to and
 // from the host); R-MAT 2^22 vertices, 2^26 edges SSSP 2.49 -> 1.01 ms (4.22
 // with another source); grid 512 x 512 22.9 -> 5.9 ms; BFS on 60,013 vertices
-// and 983,040 edges 379 -> 109 us; min labels of a symmetrised R-MAT of 2^20
+// and 983,040 edges 379 -> 107 us; min labels of a symmetrised R-MAT of 2^20
 // vertices and 2^25 edges 720 -> 281 us; 64 R-MAT graphs in one run (768,000
 // vertices, 12.3 M edges) 1.61 -> 0.72 ms.
 #pragma once
@@ -51,6 +51,13 @@ namespace kites_internal {
 constexpr int kFrThreads = 512;               // one CTA per SM, 128 registers a thread
 constexpr int kFrWarps = kFrThreads / 32;
 constexpr uint32_t kShort = 160u << 10;       // out-edges of a short iteration, at most
+// BFS turns bottom-up when the frontier has more than a third of the out-edges
+// not walked yet, and more than a short iteration's.  A third, a quarter, an
+// eighth and a twentieth took 399, 416, 448 and 518 us on R-MAT of 2^22 vertices
+// and 2^26 edges, 482, 480, 566 and 567 on an Erdos-Renyi graph of that size
+// (549 and 680 us with pushes only).
+constexpr uint32_t kBottomShare = 3;
+constexpr uint32_t kLongRow = 1024;           // in-edges one warp looks through, at most
 constexpr int kShortFlight = 2, kWideFlight = 8;  // edges in flight per lane
 constexpr int kShortCand = 2, kWideCand = 4;      // candidates a lane applies together
 constexpr uint32_t kCandRoom = 32 * (kWideCand + kWideFlight);
@@ -490,6 +497,110 @@ struct frontier_run {
     if (!kCheck) apply<kWideCand>(0);
   }
 
+  // All CTAs meet inside a step.
+  __device__ bool mid_sync() {
+    __shared__ uint32_t s_go;
+    __syncthreads();
+    if (wib == 0) {
+      const bool ok = meet();
+      if (lane == 0) s_go = ok;
+    } else {
+      ++met;
+    }
+    __syncthreads();
+    return s_go != 0u;
+  }
+
+  // BFS with the frontier at `level`: instead of relaxing its out-edges, every
+  // vertex not reached yet looks for an in-neighbour at `level`.  Where the
+  // frontier holds much of what is left to explore, most rows end at one of
+  // their first edges.  A lane looks at its vertex's first kProbe in-edges,
+  // the warp at a row's rest; what is longer than kLongRow is left to the
+  // whole grid by segment (in big[qp], which this step does not read).
+  // V is read past L1: a stale value would hide a parent.
+  __device__ bool bottom_up(uint32_t level) {
+    constexpr uint32_t kProbe = 8, kWindows = 4;
+    const uint64_t stride = (uint64_t)gridDim.x * kFrThreads;
+    const uint64_t t0 = (uint64_t)blockIdx.x * kFrThreads + threadIdx.x;
+    for (uint64_t w = t0; w < a.nwords; w += stride) queued(qp)[w] = 0u;
+    // Whether one of in-edges [r, e) comes from `level` (whole warps).
+    auto scan = [&](OffT r, OffT e) {
+      for (OffT i = r; i < e; i += 32 * kWindows) {
+        bool hit = false;
+#pragma unroll
+        for (uint32_t k = 0; k < kWindows; ++k) {
+          const OffT j = i + (OffT)(k * 32 + lane);
+          if (j < e) hit |= __ldcg(a.V + a.C[j]) == level;
+        }
+        if (lane == 0) n_relaxed += min((unsigned long long)(e - i), 32ull * kWindows);
+        if (__any_sync(kFull, hit)) return true;
+      }
+      return false;
+    };
+    for (uint64_t v0 = t0 & ~31ull; v0 < a.n; v0 += stride) {
+      const uint64_t v = v0 + lane;
+      OffT r = 0, e = 0;
+      if (v < a.n && __ldcg(a.V + v) == kInf) {
+        r = a.R[v];
+        e = a.R[v + 1];
+      }
+      if (!__any_sync(kFull, r < e)) continue;
+      bool hit = false;
+      for (uint32_t p = 0; p < kProbe; p += 4) {
+        uint32_t u[4];
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k)
+          u[k] = !hit && r + (OffT)k < e ? a.C[r + (OffT)k] : kInf;
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k) {
+          if (u[k] == kInf) continue;
+          hit |= __ldcg(a.V + u[k]) == level;
+          n_relaxed += 1;
+        }
+        if (!hit) r = e - r > (OffT)4 ? r + (OffT)4 : e;
+      }
+      const bool more = !hit && r < e;
+      uint32_t rest = __ballot_sync(kFull, more && e - r <= (OffT)kLongRow);
+      while (rest) {
+        const uint32_t src = __ffs(rest) - 1;
+        rest &= rest - 1;
+        const bool found = scan(__shfl_sync(kFull, r, src), __shfl_sync(kFull, e, src));
+        if (lane == src) hit = found;
+      }
+      for (uint32_t far = __ballot_sync(kFull, more && e - r > (OffT)kLongRow); far;
+           far &= far - 1) {
+        const uint32_t src = __ffs(far) - 1;
+        const OffT len = __shfl_sync(kFull, e - r, src);
+        const uint32_t segs = (uint32_t)((len + (OffT)(kLongRow - 1)) / (OffT)kLongRow);
+        uint32_t at = 0;
+        if (lane == 0) at = atomicAdd(&cur()->bticket, segs);
+        at = __shfl_sync(kFull, at, 0);
+        for (uint32_t i = lane; i < segs; i += 32)
+          a.big[qp][at + i] = make_uint2((uint32_t)(v0 + src), i);
+      }
+      uint32_t deg = 0;
+      if (hit) {
+        a.V[v] = level + 1u;
+        deg = a.out_deg[v];
+        n_updated += 1;
+      }
+      if (__any_sync(kFull, hit)) push(hit, false, (uint32_t)v, deg, fc, far_c);
+    }
+    if (!mid_sync()) return false;
+    const uint32_t segs = __ldcg(&cur()->bticket);
+    for (uint32_t i = wib * gridDim.x + blockIdx.x; i < segs; i += gridDim.x * kFrWarps) {
+      const uint2 en = __ldcg(a.big[qp] + i);
+      if (__ldcg(a.V + en.x) != kInf) continue;
+      const OffT r = a.R[en.x] + (OffT)kProbe + (OffT)en.y * kLongRow, e = a.R[en.x + 1];
+      if (!scan(r, e - r > (OffT)kLongRow ? r + (OffT)kLongRow : e)) continue;
+      bool mine = false;
+      if (lane == 0) mine = atomicMin(a.V + en.x, level + 1u) == kInf;
+      if (lane == 0 && mine) n_updated += 1;
+      push(mine, false, en.x, a.out_deg[en.x], fc, far_c);
+    }
+    return true;
+  }
+
   // Queues every vertex for which on(v).
   template <class Pred>
   __device__ void seed_all(Pred on) {
@@ -696,8 +807,14 @@ struct frontier_run {
         ++bucket_rounds;
         bucket_edges += sl.edges;
         spent += sl.edges;
-        if (sl.edges <= kShort) short_push(sl);
-        else wide_push<false>(sl);
+        if (OP == OP_BFS && a.seed != kSeedFinite && sl.edges > kShort &&
+            sl.edges > (a.m + sl.edges - spent) / kBottomShare) {
+          if (!bottom_up(rounds - 1u)) return finish(false, true);
+        } else if (sl.edges <= kShort) {
+          short_push(sl);
+        } else {
+          wide_push<false>(sl);
+        }
         if (!end(fc, far_c)) return finish(false, true);
       }
       qp ^= 1u;

@@ -90,6 +90,36 @@ def test_wide_iterations(engine, scale, factor):
         g.close()
 
 
+@pytest.mark.parametrize("offsets64", [False, True])
+@pytest.mark.parametrize("deg", [3, 4, 5, 8, 9, 40, 1031, 1032, 1033, 5000])
+def test_bottom_up_rows(engine, deg, offsets64):
+    """BFS whose second frontier holds most of the edges, so that unreached
+    vertices look for a parent: rows of `deg` in-edges whose only parent is
+    their last in-neighbour, or that have none."""
+    n, mids = 60000, np.arange(57000, 60000, dtype=np.uint32)
+    rng = np.random.default_rng(deg)
+    far = np.arange(1, 20000, dtype=np.uint32)            # never reached
+    s = [np.zeros(mids.shape[0], np.uint32), np.repeat(mids, 100)]
+    d = [mids, rng.integers(31000, 57000, 100 * mids.shape[0], dtype=np.uint32)]
+    for i, row in enumerate(range(30000, 30010)):
+        src = rng.choice(far, deg, replace=False)
+        if i % 2:
+            src[-1] = mids[7 * i]
+        s.append(src)
+        d.append(np.full(deg, row, np.uint32))
+    s.append(np.arange(30000, 30010, dtype=np.uint32))    # and one level below
+    d.append(np.arange(30500, 30510, dtype=np.uint32))
+    s, d = np.concatenate(s), np.concatenate(d)
+    R, C, _ = capi.csc_from_edges(n, s, d)
+    g = capi.Graph(engine, R, C, None, offsets64=offsets64)
+    try:
+        dist, _ = g.sssp(0, op=capi.OP_BFS)
+        np.testing.assert_array_equal(dist, oracle(R, C, None, n, [0], O.OP_BFS_SAT))
+        assert dist[30001] == 2 and dist[30000] == INF and dist[30501] == 3
+    finally:
+        g.close()
+
+
 @pytest.mark.parametrize("op,oop", OPS + [(capi.OP_CC, None)])
 @pytest.mark.parametrize("state", ["sources", "missing", "partial", "empty", "settled"])
 def test_process_states(engine, op, oop, state):
