@@ -9,6 +9,7 @@
 
 #include <algorithm>
 #include <chrono>
+#include <type_traits>
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
 
@@ -18,6 +19,7 @@
 #include "kernels_batch.cuh"
 #include "kernels_batch_async.cuh"
 #include "kernels_batch_tma.cuh"
+#include "kernels_build.cuh"
 #include "kernels_mip.cuh"
 #include "kernels_pr.cuh"
 #include "kernels_select.cuh"
@@ -88,6 +90,13 @@ int graph_alloc(kites_graph *g, void **p, size_t bytes) {
   KITES_TRY(dev_alloc(g->eng, p, bytes));
   g->owned.push_back(*p);
   return KITES_OK;
+}
+
+void graph_release(kites_graph *g, void *p) {
+  if (!p) return;
+  cudaFreeAsync(p, g->eng->stream);
+  auto &o = g->owned;
+  o.erase(std::remove(o.begin(), o.end(), p), o.end());
 }
 
 inline unsigned grid_for(uint64_t n, unsigned block = 256, unsigned cap = 65535u * 8) {
@@ -173,7 +182,8 @@ int validate_csc(kites_graph *g, const OffT *R, uint64_t n_rows, uint64_t n_edge
   uint32_t *bad = (uint32_t *)p;
   KITES_CUDA_TRY(cudaMemsetAsync(bad, 0, 4, s));
   if (n_rows) k_validate_rows<OffT><<<grid_for(n_rows), 256, 0, s>>>(R, n_rows, n_edges, bad);
-  if (n_edges) k_validate_ids<<<grid_for(n_edges), 256, 0, s>>>(ids, n_edges, limit, bad);
+  if (n_edges) 
+    k_validate_ids<<<grid_for(n_edges / 4 + 1, 256, 2048), 256, 0, s>>>(ids, n_edges, limit, bad);
   KITES_CUDA_TRY(cudaGetLastError());
   uint32_t *h = (uint32_t *)eng->pinned;
   KITES_CUDA_TRY(cudaMemcpyAsync(h, bad, 4, cudaMemcpyDeviceToHost, s));
@@ -186,14 +196,71 @@ int validate_csc(kites_graph *g, const OffT *R, uint64_t n_rows, uint64_t n_edge
   return KITES_OK;
 }
 
-// Weighted vertex-level out-CSR from the CSC: stable radix sort of the edge
-// indices by source keeps destinations ascending within each out-row.
+// Grid of the construction kernels: `per` edges a thread, 256 threads.
+unsigned grid_of_edges(uint64_t m, unsigned per) {
+  return (unsigned)((m + 256ull * per - 1) / (256ull * per));
+}
+
+int bits_for(uint64_t n) {
+  int b = 1;
+  while (b < 32 && (1ull << b) < n) ++b;
+  return b;
+}
+
+// Offsets [n + 1] from the rows' ends (as mark_ends leaves them, n + 1 zeroed
+// entries each), and the row lengths into deg if it is not null.
 template <typename OffT>
-int build_out_csr(kites_graph *g) {
+int scan_row_ends(kites_engine *eng, const uint32_t *first, const uint32_t *last, uint64_t n,
+                  OffT *R, uint32_t *deg) {
+  cudaStream_t s = eng->stream;
+  void *wide, *temp;
+  KITES_TRY(dev_alloc(eng, &wide, (n + 1) * sizeof(OffT)));
+  k_row_lengths<OffT><<<grid_for(n + 1), 256, 0, s>>>(first, last, n + 1, (OffT *)wide, deg);
+  size_t temp_bytes = 0;
+  KITES_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, temp_bytes, (OffT *)wide, R,
+                                               (uint64_t)(n + 1), s));
+  KITES_TRY(dev_alloc(eng, &temp, temp_bytes));
+  KITES_CUDA_TRY(cub::DeviceScan::ExclusiveSum(temp, temp_bytes, (OffT *)wide, R,
+                                               (uint64_t)(n + 1), s));
+  KITES_CUDA_TRY(cudaFreeAsync(temp, s));
+  KITES_CUDA_TRY(cudaFreeAsync(wide, s));
+  return KITES_OK;
+}
+
+// Sorts (source, payload) pairs of the CSC by source, stably, and unpacks them
+// into outC, outE and the sources' row ends.
+template <typename PayT>
+int transpose_edges(kites_graph *g, const PayT *pay, uint32_t *ends) {
   kites_engine *eng = g->eng;
   cudaStream_t s = eng->stream;
   const uint64_t n = g->n, m = g->m;
-  const OffT *R = (const OffT *)g->R;
+  void *keys, *pays, *temp;
+  KITES_TRY(dev_alloc(eng, &keys, m * 4));
+  KITES_TRY(dev_alloc(eng, &pays, m * sizeof(PayT)));
+  size_t temp_bytes = 0;
+  const int bits = bits_for(n);
+  KITES_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, temp_bytes, g->C, (uint32_t *)keys, pay,
+                                                 (PayT *)pays, (uint64_t)m, 0, bits, s));
+  KITES_TRY(dev_alloc(eng, &temp, temp_bytes));
+  KITES_CUDA_TRY(cub::DeviceRadixSort::SortPairs(temp, temp_bytes, g->C, (uint32_t *)keys, pay,
+                                                 (PayT *)pays, (uint64_t)m, 0, bits, s));
+  k_unpack_edges<PayT><<<grid_of_edges(m, kBuildPer), 256, 0, s>>>(
+      (const uint32_t *)keys, (const PayT *)pays, m, g->outC, g->outE, ends, ends + n + 1);
+  KITES_CUDA_TRY(cudaGetLastError());
+  KITES_CUDA_TRY(cudaFreeAsync(temp, s));
+  KITES_CUDA_TRY(cudaFreeAsync(pays, s));
+  KITES_CUDA_TRY(cudaFreeAsync(keys, s));
+  return KITES_OK;
+}
+
+// Weighted vertex-level out-CSR from the CSC: stable radix sort of the edges
+// by source keeps destinations ascending within each out-row.  `row` is the
+// row of every edge.
+template <typename OffT>
+int build_out_csr(kites_graph *g, const uint32_t *row) {
+  kites_engine *eng = g->eng;
+  cudaStream_t s = eng->stream;
+  const uint64_t n = g->n, m = g->m;
   void *p;
   KITES_TRY(graph_alloc(g, &p, (n + 1) * sizeof(OffT)));
   g->outR = p;
@@ -203,77 +270,69 @@ int build_out_csr(kites_graph *g) {
   g->outE = (uint32_t *)p;
   KITES_TRY(graph_alloc(g, &p, (n + 1) * sizeof(uint32_t)));
   g->out_deg = (uint32_t *)p;
-  KITES_CUDA_TRY(cudaMemsetAsync(g->out_deg, 0, (n + 1) * sizeof(uint32_t), s));
-  // The transposition sorts 32-bit edge ids (item counts are 64-bit).
+  // Row ends are 32-bit edge numbers.
   if (m > 0xFFFFFFFFull)
     return fail(KITES_ERR_UNSUPPORTED, "out-CSR build supports < 2^32 edges");
-  if (m) {
-    k_count_u32<<<grid_for(m), 256, 0, s>>>(g->C, m, g->out_deg);
-    KITES_CUDA_TRY(cudaGetLastError());
+  KITES_TRY(dev_alloc(eng, &p, 2 * (n + 1) * sizeof(uint32_t)));
+  uint32_t *ends = (uint32_t *)p;
+  KITES_CUDA_TRY(cudaMemsetAsync(ends, 0, 2 * (n + 1) * sizeof(uint32_t), s));
+  if (m && g->esize == 4) {
+    KITES_TRY(dev_alloc(eng, &p, m * 8));
+    k_pack_edges<<<grid_of_edges(m, kBuildPer), 256, 0, s>>>(row, (const uint32_t *)g->E, m,
+                                                            (uint64_t *)p);
+    KITES_TRY(transpose_edges<uint64_t>(g, (const uint64_t *)p, ends));
+    KITES_CUDA_TRY(cudaFreeAsync(p, s));
+  } else if (m) {
+    KITES_TRY(transpose_edges<uint32_t>(g, row, ends));
   }
-  // outR = exclusive scan of out-degrees (as OffT).
-  OffT *deg_wide;
-  KITES_TRY(dev_alloc(eng, &p, (n + 1) * sizeof(OffT)));
-  deg_wide = (OffT *)p;
-  k_widen_offsets<OffT><<<grid_for(n + 1), 256, 0, s>>>(g->out_deg, n + 1, deg_wide);
-  size_t temp_bytes = 0;
-  KITES_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, temp_bytes, deg_wide,
-                                               (OffT *)g->outR, (uint64_t)(n + 1), s));
-  void *temp;
-  KITES_TRY(dev_alloc(eng, &temp, temp_bytes));
-  KITES_CUDA_TRY(cub::DeviceScan::ExclusiveSum(temp, temp_bytes, deg_wide,
-                                               (OffT *)g->outR, (uint64_t)(n + 1), s));
-  KITES_CUDA_TRY(cudaFreeAsync(temp, s));
-  KITES_CUDA_TRY(cudaFreeAsync(deg_wide, s));
-  if (m == 0) return KITES_OK;
-
-  uint32_t *row, *keys_out, *idx_in, *idx_out;
-  KITES_TRY(dev_alloc(eng, &p, m * 4)); row = (uint32_t *)p;
-  KITES_TRY(dev_alloc(eng, &p, m * 4)); keys_out = (uint32_t *)p;
-  KITES_TRY(dev_alloc(eng, &p, m * 4)); idx_in = (uint32_t *)p;
-  KITES_TRY(dev_alloc(eng, &p, m * 4)); idx_out = (uint32_t *)p;
-  k_row_of_edge<OffT><<<grid_for(m), 256, 0, s>>>(R, n + 1, m, row);
-  k_iota_u32<<<grid_for(m), 256, 0, s>>>(idx_in, m);
-  KITES_CUDA_TRY(cudaGetLastError());
-  int end_bit = 1;
-  while (end_bit < 32 && (1ull << end_bit) < n) ++end_bit;
-  temp_bytes = 0;
-  KITES_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, temp_bytes, g->C, keys_out,
-                                                 idx_in, idx_out, (uint64_t)m, 0, end_bit, s));
-  KITES_TRY(dev_alloc(eng, &temp, temp_bytes));
-  KITES_CUDA_TRY(cub::DeviceRadixSort::SortPairs(temp, temp_bytes, g->C, keys_out,
-                                                 idx_in, idx_out, (uint64_t)m, 0, end_bit, s));
-  k_gather_out<OffT><<<grid_for(m), 256, 0, s>>>(
-      idx_out, row, g->esize == 4 ? (const uint32_t *)g->E : nullptr, m, g->outC, g->outE);
-  KITES_CUDA_TRY(cudaGetLastError());
-  KITES_CUDA_TRY(cudaFreeAsync(temp, s));
-  KITES_CUDA_TRY(cudaFreeAsync(row, s));
-  KITES_CUDA_TRY(cudaFreeAsync(keys_out, s));
-  KITES_CUDA_TRY(cudaFreeAsync(idx_in, s));
-  KITES_CUDA_TRY(cudaFreeAsync(idx_out, s));
+  KITES_TRY(scan_row_ends<OffT>(eng, ends, ends + n + 1, n, (OffT *)g->outR, g->out_deg));
+  KITES_CUDA_TRY(cudaFreeAsync(ends, s));
   return KITES_OK;
 }
 
+// Arrays of a CSC that were built on the device, which the graph takes over:
+// offsets of the graph's own type, padded; checked; the row of every edge.
+struct built_csc {
+  void *R = nullptr;
+  uint32_t *C = nullptr, *E = nullptr, *rowid = nullptr;
+};
+
 template <typename OffT>
-int upload_typed(kites_graph *g, const kites_csc_view *v) {
+int upload_typed(kites_graph *g, const kites_csc_view *v, const built_csc *built) {
   kites_engine *eng = g->eng;
   cudaStream_t s = eng->stream;
-  OffT *R;
-  KITES_TRY(upload_offsets<OffT>(g, v->row_offsets, v->row_offsets32, v->n_vertices,
-                                 g->n, v->on_device, &R));
-  g->R = R;
   void *p;
-  KITES_TRY(graph_alloc(g, &p, g->m * sizeof(uint32_t)));
-  g->C = (uint32_t *)p;
-  if (g->m)
-    KITES_CUDA_TRY(cudaMemcpyAsync(g->C, v->col_indices, g->m * 4, cudaMemcpyDefault, s));
-  KITES_TRY(validate_csc<OffT>(g, R, g->n, g->m, g->C, g->n_given, "CSC"));
-  if (g->esize) {
-    KITES_TRY(graph_alloc(g, &p, g->m * g->esize));
-    g->E = p;
+  uint32_t *row = nullptr;
+  if (built) {
+    g->R = built->R;
+    g->C = built->C;
+    g->E = built->E;
+    row = built->rowid;
+    for (void *q : {(void *)g->R, (void *)g->C, (void *)g->E, (void *)row})
+      if (q) g->owned.push_back(q);
+  } else {
+    OffT *R;
+    KITES_TRY(upload_offsets<OffT>(g, v->row_offsets, v->row_offsets32, v->n_vertices,
+                                   g->n, v->on_device, &R));
+    g->R = R;
+    KITES_TRY(graph_alloc(g, &p, g->m * sizeof(uint32_t)));
+    g->C = (uint32_t *)p;
     if (g->m)
-      KITES_CUDA_TRY(cudaMemcpyAsync(g->E, v->edge_values, g->m * g->esize,
-                                     cudaMemcpyDefault, s));
+      KITES_CUDA_TRY(cudaMemcpyAsync(g->C, v->col_indices, g->m * 4, cudaMemcpyDefault, s));
+    KITES_TRY(validate_csc<OffT>(g, R, g->n, g->m, g->C, g->n_given, "CSC"));
+    if (g->esize) {
+      KITES_TRY(graph_alloc(g, &p, g->m * g->esize));
+      g->E = p;
+      if (g->m)
+        KITES_CUDA_TRY(cudaMemcpyAsync(g->E, v->edge_values, g->m * g->esize,
+                                       cudaMemcpyDefault, s));
+    }
+    if (g->m) {
+      KITES_TRY(graph_alloc(g, &p, g->m * 4));
+      row = (uint32_t *)p;
+      k_row_of_edge<OffT><<<grid_of_edges(g->m, 8), 256, 0, s>>>(R, g->n + 1, g->m, row);
+      KITES_CUDA_TRY(cudaGetLastError());
+    }
   }
   KITES_TRY(graph_alloc(g, &p, g->n * g->vsize));
   g->V = p;
@@ -284,7 +343,7 @@ int upload_typed(kites_graph *g, const kites_csc_view *v) {
 
   // Out-CSR structure for every graph; its weights only mean something for
   // 4-byte edge values (other sizes get 1).
-  KITES_TRY(build_out_csr<OffT>(g));
+  KITES_TRY(build_out_csr<OffT>(g, row));
 
   // Activation adjacency.
   if (!g->directed) {
@@ -341,14 +400,7 @@ int upload_typed(kites_graph *g, const kites_csc_view *v) {
 
   // Edge-parallel dense sweeps: the row of every edge, persistent grid.
   if (g->vpg == 1) {
-    if (g->m) {
-      void *p;
-      KITES_TRY(graph_alloc(g, &p, g->m * 4));
-      g->rowid = (uint32_t *)p;
-      k_row_of_edge<OffT><<<grid_for(g->m), 256, 0, eng->stream>>>((const OffT *)g->R, g->n + 1,
-                                                                  g->m, g->rowid);
-      KITES_CUDA_TRY(cudaGetLastError());
-    }
+    g->rowid = row;
     int per_sm_sweep = 0;
     KITES_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
         &per_sm_sweep, k_sweep<OP_SSSP, OffT, kRowFilter>, kSweepThreads, 0));
@@ -358,6 +410,8 @@ int upload_typed(kites_graph *g, const kites_csc_view *v) {
     g->sweep_grid = (int)std::max<uint64_t>(1, std::min<uint64_t>(want_blocks, scap));
     g->dense_edges = g->m / 16;
     g->dense_rows = g->n / 32;
+  } else {
+    graph_release(g, row);
   }
   return KITES_OK;
 }
@@ -716,8 +770,8 @@ int run_pagerank(kites_graph *g, uint64_t n_real, float *out, const kites_run_op
   if (!g->rowid && !g->pr_rowid && g->m) {   // vertex groups have no sweeps' row index
     KITES_TRY(graph_alloc(g, &p, g->m * 4));
     g->pr_rowid = (uint32_t *)p;
-    k_row_of_edge<OffT><<<grid_for(g->m), 256, 0, s>>>((const OffT *)g->R, g->n + 1, g->m,
-                                                      g->pr_rowid);
+    k_row_of_edge<OffT><<<grid_of_edges(g->m, 8), 256, 0, s>>>((const OffT *)g->R, g->n + 1,
+                                                              g->m, g->pr_rowid);
   }
   float *x[2] = {g->pr_x, g->pr_x + g->n};
   float *pr = (float *)g->V, *inv_out = g->pr_x + 3 * g->n;
@@ -1325,13 +1379,6 @@ int dispatch_record(kites_graph *g, int op, float *feat, float *times, uint32_t 
 }
 
 // ---- batched multi-source runs -------------------------------------------
-
-void graph_release(kites_graph *g, void *p) {
-  if (!p) return;
-  cudaFreeAsync(p, g->eng->stream);
-  auto &o = g->owned;
-  o.erase(std::remove(o.begin(), o.end(), p), o.end());
-}
 
 void drop_batch_loops(kites_graph *g) {
   for (auto it = g->loops.begin(); it != g->loops.end();) {
@@ -2323,6 +2370,9 @@ extern "C" int kites_graph_destroy(kites_graph *g) {
   return KITES_OK;
 }
 
+static int upload_graph(kites_engine *eng, const kites_csc_view *v, const built_csc *built,
+                        kites_graph **out);
+
 extern "C" int kites_graph_upload(kites_engine *eng, const kites_csc_view *v,
                                   kites_graph **out) {
   clear_error();
@@ -2341,6 +2391,14 @@ extern "C" int kites_graph_upload(kites_engine *eng, const kites_csc_view *v,
   if (v->edge_value_size && !v->edge_values && v->n_edges)
     return fail(KITES_ERR_INVALID, "edge_value_size set but no edge values");
   KITES_TRY(set_device(eng));
+  return upload_graph(eng, v, nullptr, out);
+}
+
+// The graph of a checked view, or of arrays built on the device (the view then
+// has the sizes only); those are the graph's whatever the outcome.
+static int upload_graph(kites_engine *eng, const kites_csc_view *v, const built_csc *built,
+                        kites_graph **out) {
+  const uint32_t vpg = v->vertex_per_group ? v->vertex_per_group : 1;
   kites_graph *g = new kites_graph();
   g->eng = eng;
   eng->graphs.push_back(g);
@@ -2353,7 +2411,7 @@ extern "C" int kites_graph_upload(kites_engine *eng, const kites_csc_view *v,
   g->off64 = v->offsets64 != 0 || g->m > 0xFFFFFFFFull - g->n;
   g->vsize = v->vertex_value_size ? v->vertex_value_size : 4;
   g->esize = v->edge_value_size;
-  int st = g->off64 ? upload_typed<uint64_t>(g, v) : upload_typed<uint32_t>(g, v);
+  int st = g->off64 ? upload_typed<uint64_t>(g, v, built) : upload_typed<uint32_t>(g, v, built);
   void *p = nullptr;
   if (st == KITES_OK) {
     g->nbits = (g->n + vpg - 1) / vpg;
@@ -2398,38 +2456,97 @@ extern "C" int kites_graph_upload(kites_engine *eng, const kites_csc_view *v,
 
 // ---- device-side ingestion (edge list -> CSC) -----------------------------
 
-// keys[i] = dst << 32 | src; any endpoint >= n sets *bad.
-__global__ void k_edge_keys(const uint32_t *__restrict__ src, const uint32_t *__restrict__ dst,
-                            uint64_t m, uint64_t n, uint64_t *__restrict__ keys, uint32_t *bad) {
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m;
-       i += (uint64_t)gridDim.x * blockDim.x) {
-    const uint32_t s = src[i], d = dst[i];
-    if (s >= n || d >= n) atomicOr(bad, 1u);
-    keys[i] = (uint64_t)d << 32 | s;
+// An array the caller gave, as device memory: itself, or a copy in *tmp.
+static int on_device(kites_engine *eng, const uint32_t *p, uint64_t m, const uint32_t **out,
+                     std::vector<void *> *tmp) {
+  cudaPointerAttributes attr;
+  const bool dev = cudaPointerGetAttributes(&attr, p) == cudaSuccess &&
+                   attr.type == cudaMemoryTypeDevice && attr.device == eng->device;
+  cudaGetLastError();
+  if (dev) {
+    *out = p;
+    return KITES_OK;
   }
+  void *q;
+  KITES_TRY(dev_alloc(eng, &q, m * 4));
+  tmp->push_back(q);
+  KITES_CUDA_TRY(cudaMemcpyAsync(q, p, m * 4, cudaMemcpyDefault, eng->stream));
+  *out = (const uint32_t *)q;
+  return KITES_OK;
 }
 
-// R[d] = first sorted edge whose destination is >= d (binary search), for
-// d in [0, n]; C[i] = source of sorted edge i.
-__global__ void k_rows_of_keys(const uint64_t *__restrict__ keys, uint64_t m, uint64_t n,
-                               uint64_t *__restrict__ R, uint32_t *__restrict__ C) {
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t d = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; d <= n; d += stride) {
-    uint64_t lo = 0, hi = m;  // first index with key >> 32 >= d
-    while (lo < hi) {
-      const uint64_t mid = (lo + hi) >> 1;
-      if ((keys[mid] >> 32) < d) lo = mid + 1; else hi = mid;
-    }
-    R[d] = lo;
+// Sorts the edges by (destination, source), stably, and builds the CSC arrays
+// the graph takes over.  KeyT holds destination << bits | source; what a sort
+// of it costs goes with its bits, so they are no more than n needs.
+template <typename KeyT, typename OffT>
+static int build_csc(kites_engine *eng, uint64_t n, uint64_t n_padded, uint64_t m,
+                     const uint32_t *src, const uint32_t *dst, const uint32_t *weights, int bits,
+                     built_csc *b, std::vector<void *> *tmp) {
+  cudaStream_t s = eng->stream;
+  auto alloc = [&](auto **q, size_t bytes) {
+    void *p = nullptr;
+    const int st = dev_alloc(eng, &p, bytes);
+    if (st == KITES_OK) tmp->push_back(p);
+    *q = (std::remove_reference_t<decltype(**q)> *)p;
+    return st;
+  };
+  auto drop = [&](void *p) {
+    cudaFreeAsync(p, s);
+    tmp->erase(std::remove(tmp->begin(), tmp->end(), p), tmp->end());
+  };
+  const uint64_t mm = std::max<uint64_t>(m, 1);
+  uint32_t *bad, *ends;
+  KITES_TRY(alloc(&bad, 4));
+  KITES_TRY(alloc(&ends, 2 * (n_padded + 1) * 4));
+  KITES_CUDA_TRY(cudaMemsetAsync(bad, 0, 4, s));
+  KITES_CUDA_TRY(cudaMemsetAsync(ends, 0, 2 * (n_padded + 1) * 4, s));
+  OffT *R;
+  KITES_TRY(alloc(&R, (n_padded + 1) * sizeof(OffT)));
+  KITES_TRY(alloc(&b->C, mm * 4));
+  KITES_TRY(alloc(&b->rowid, mm * 4));
+  b->R = R;
+  if (weights) KITES_TRY(alloc(&b->E, mm * 4));
+  if (m) {
+    KeyT *keys, *sorted;
+    char *temp;
+    KITES_TRY(alloc(&keys, m * sizeof(KeyT)));
+    KITES_TRY(alloc(&sorted, m * sizeof(KeyT)));
+    const unsigned grid = grid_of_edges(m, kBuildPer);
+    if (((uintptr_t)src | (uintptr_t)dst) % 16 == 0)
+      k_edge_keys<KeyT, true><<<grid, 256, 0, s>>>(src, dst, m, n, bits, keys, bad);
+    else
+      k_edge_keys<KeyT, false><<<grid, 256, 0, s>>>(src, dst, m, n, bits, keys, bad);
+    KITES_CUDA_TRY(cudaGetLastError());
+    uint32_t *hbad = (uint32_t *)eng->pinned;
+    KITES_CUDA_TRY(cudaMemcpyAsync(hbad, bad, 4, cudaMemcpyDeviceToHost, s));
+    KITES_CUDA_TRY(cudaStreamSynchronize(s));
+    if (*hbad) return fail(KITES_ERR_INVALID, "edge endpoint >= n_vertices");
+    size_t bytes = 0;
+    auto sort = [&](void *t) {
+      return weights ? cub::DeviceRadixSort::SortPairs(t, bytes, keys, sorted, weights, b->E,
+                                                       (uint64_t)m, 0, 2 * bits, s)
+                     : cub::DeviceRadixSort::SortKeys(t, bytes, keys, sorted, (uint64_t)m, 0,
+                                                      2 * bits, s);
+    };
+    KITES_CUDA_TRY(sort(nullptr));
+    KITES_TRY(alloc(&temp, bytes));
+    KITES_CUDA_TRY(sort(temp));
+    k_split_keys<KeyT><<<grid, 256, 0, s>>>(sorted, m, bits, b->C, b->rowid, ends,
+                                            ends + n_padded + 1);
+    KITES_CUDA_TRY(cudaGetLastError());
+    // The keys and the sort's scratch go back to the pool before the upload
+    // builds the out-CSR: at 2^31 edges that is about 50 GB less at the peak.
+    drop(keys);
+    drop(sorted);
+    drop(temp);
   }
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += stride)
-    C[i] = (uint32_t)keys[i];
+  return scan_row_ends<OffT>(eng, ends, ends + n_padded + 1, n_padded, R, nullptr);
 }
 
 // Builds the CSC of an edge list on the device -- rows keyed by
 // destination, each row's sources ascending, parallel edges kept in input
-// order (a stable radix sort of dst << 32 | src) -- and uploads it as
-// kites_graph_upload does.  The edge arrays may be host or device memory.
+// order (a stable radix sort) -- and the graph over it, as kites_graph_upload
+// does.  The edge arrays may be host or device memory.
 extern "C" int kites_graph_from_edges(kites_engine *eng, uint64_t n_vertices, uint64_t n_edges,
                                       const uint32_t *src, const uint32_t *dst,
                                       const uint32_t *weights, int directed,
@@ -2444,95 +2561,41 @@ extern "C" int kites_graph_from_edges(kites_engine *eng, uint64_t n_vertices, ui
     return fail(KITES_ERR_UNSUPPORTED, "device ingestion takes < 2^32 edges");
   KITES_TRY(set_device(eng));
   cudaStream_t s = eng->stream;
-  const uint64_t m = n_edges, n = n_vertices;
-  void *p = nullptr;
-  uint64_t *keys[2] = {nullptr, nullptr}, *R = nullptr;
-  uint32_t *ends[2] = {nullptr, nullptr}, *w[2] = {nullptr, nullptr}, *C = nullptr, *bad = nullptr;
-  void *temp = nullptr;
+  const uint64_t m = n_edges, n = n_vertices, n_padded = (n + 127) / 128 * 128;
+  const int bits = bits_for(n);
+  const bool off64 = m > 0xFFFFFFFFull - n_padded, wide = bits > 16;
   std::vector<void *> tmp;
-  auto alloc = [&](void **q, size_t bytes) {
-    int st = dev_alloc(eng, q, bytes);
-    if (st == KITES_OK) tmp.push_back(*q);
-    return st;
-  };
+  built_csc b;
   int st = KITES_OK;
-  do {
-    const size_t mm = (size_t)std::max<uint64_t>(m, 1);
-    if ((st = alloc(&p, mm * 8)) != KITES_OK) break;
-    keys[0] = (uint64_t *)p;
-    if ((st = alloc(&p, mm * 8)) != KITES_OK) break;
-    keys[1] = (uint64_t *)p;
-    if ((st = alloc(&p, (n + 1) * 8)) != KITES_OK) break;
-    R = (uint64_t *)p;
-    if ((st = alloc(&p, mm * 4)) != KITES_OK) break;
-    C = (uint32_t *)p;
-    if ((st = alloc(&p, 4)) != KITES_OK) break;
-    bad = (uint32_t *)p;
-    if (weights) {
-      if ((st = alloc(&p, mm * 4)) != KITES_OK) break;
-      w[0] = (uint32_t *)p;
-      if ((st = alloc(&p, mm * 4)) != KITES_OK) break;
-      w[1] = (uint32_t *)p;
-    }
-    cudaError_t e = cudaMemsetAsync(bad, 0, 4, s);
-    if (m) {
-      // The endpoints pass through the second key buffer (2 x 4 bytes an edge).
-      ends[0] = (uint32_t *)keys[1];
-      ends[1] = ends[0] + m;
-      if (e == cudaSuccess) e = cudaMemcpyAsync(ends[0], src, m * 4, cudaMemcpyDefault, s);
-      if (e == cudaSuccess) e = cudaMemcpyAsync(ends[1], dst, m * 4, cudaMemcpyDefault, s);
-      if (e == cudaSuccess && weights)
-        e = cudaMemcpyAsync(w[0], weights, m * 4, cudaMemcpyDefault, s);
-      if (e != cudaSuccess) { st = fail(KITES_ERR_CUDA, "edge copy: %s", cudaGetErrorString(e)); break; }
-      k_edge_keys<<<grid_for(m), 256, 0, s>>>(ends[0], ends[1], m, n, keys[0], bad);
-      uint32_t hbad = 0;
-      e = cudaMemcpyAsync(&hbad, bad, 4, cudaMemcpyDeviceToHost, s);
-      if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-      if (e != cudaSuccess) { st = fail(KITES_ERR_CUDA, "edge keys: %s", cudaGetErrorString(e)); break; }
-      if (hbad) { st = fail(KITES_ERR_INVALID, "edge endpoint >= n_vertices"); break; }
-      int end_bit = 33;
-      while (end_bit < 64 && (1ull << (end_bit - 32)) < n) ++end_bit;
-      size_t temp_bytes = 0;
-      if (weights)
-        e = cub::DeviceRadixSort::SortPairs(nullptr, temp_bytes, keys[0], keys[1], w[0], w[1],
-                                            (uint64_t)m, 0, end_bit, s);
-      else
-        e = cub::DeviceRadixSort::SortKeys(nullptr, temp_bytes, keys[0], keys[1], (uint64_t)m, 0,
-                                           end_bit, s);
-      if (e != cudaSuccess) { st = fail(KITES_ERR_CUDA, "sort: %s", cudaGetErrorString(e)); break; }
-      if ((st = alloc(&temp, temp_bytes)) != KITES_OK) break;
-      if (weights)
-        e = cub::DeviceRadixSort::SortPairs(temp, temp_bytes, keys[0], keys[1], w[0], w[1],
-                                            (uint64_t)m, 0, end_bit, s);
-      else
-        e = cub::DeviceRadixSort::SortKeys(temp, temp_bytes, keys[0], keys[1], (uint64_t)m, 0,
-                                           end_bit, s);
-      if (e != cudaSuccess) { st = fail(KITES_ERR_CUDA, "sort: %s", cudaGetErrorString(e)); break; }
-    }
-    k_rows_of_keys<<<grid_for(n + 1), 256, 0, s>>>(keys[1], m, n, R, C);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) { st = fail(KITES_ERR_CUDA, "rows: %s", cudaGetErrorString(e)); break; }
-    // The keys (16 bytes an edge), the unsorted weights and the sort's
-    // scratch go back to the pool before the upload builds the graph's own
-    // arrays: at 2^31 edges that is about 50 GB less at the peak.
-    for (void *q : {(void *)keys[0], (void *)keys[1], (void *)w[0], temp}) {
-      if (!q) continue;
-      cudaFreeAsync(q, s);
+  if (m) st = on_device(eng, src, m, &src, &tmp);
+  if (m && st == KITES_OK) st = on_device(eng, dst, m, &dst, &tmp);
+  const uint32_t *w = m ? weights : nullptr;
+  if (w && st == KITES_OK) st = on_device(eng, w, m, &w, &tmp);
+  if (weights && !m) w = weights;   // no edges, but a graph with edge values
+  if (st == KITES_OK) {
+    if (off64)
+      st = build_csc<uint64_t, uint64_t>(eng, n, n_padded, m, src, dst, w, bits, &b, &tmp);
+    else if (wide)
+      st = build_csc<uint64_t, uint32_t>(eng, n, n_padded, m, src, dst, w, bits, &b, &tmp);
+    else
+      st = build_csc<uint32_t, uint32_t>(eng, n, n_padded, m, src, dst, w, bits, &b, &tmp);
+  }
+  if (st == KITES_OK) {
+    for (void *q : {b.R, (void *)b.C, (void *)b.E, (void *)b.rowid})
       tmp.erase(std::remove(tmp.begin(), tmp.end(), q), tmp.end());
-    }
+    // The copied edge list is not needed any more.
+    for (void *q : tmp) cudaFreeAsync(q, s);
+    tmp.clear();
     kites_csc_view v = {};
     v.n_vertices = n;
     v.n_edges = m;
-    v.row_offsets = R;
-    v.col_indices = C;
-    v.edge_values = weights ? w[1] : nullptr;
     v.edge_value_size = weights ? 4 : 0;
     v.vertex_value_size = 4;
     v.vertex_per_group = 1;
     v.directed = directed ? 1 : 0;
     v.on_device = 1;
-    st = kites_graph_upload(eng, &v, out);
-  } while (0);
+    st = upload_graph(eng, &v, &b, out);
+  }
   for (void *q : tmp) cudaFreeAsync(q, s);
   cudaError_t e = cudaStreamSynchronize(s);
   if (st == KITES_OK && e != cudaSuccess)

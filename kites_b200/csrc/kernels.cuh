@@ -512,11 +512,18 @@ __global__ void k_validate_rows(const OffT *__restrict__ R, uint64_t n_rows,
   }
 }
 
+// ids: 16-byte aligned (the graph's own arrays are).
 __global__ void k_validate_ids(const uint32_t *__restrict__ ids, uint64_t n,
                                uint64_t limit, uint32_t *bad) {
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (uint64_t)gridDim.x * blockDim.x)
-    if (ids[i] >= limit) atomicOr(bad, 2u);
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  const uint64_t t0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  uint32_t top = 0;
+  for (uint64_t i = t0; i < n / 4; i += stride) {
+    const uint4 x = __ldcs(reinterpret_cast<const uint4 *>(ids) + i);
+    top = max(max(top, max(x.x, x.y)), max(x.z, x.w));
+  }
+  for (uint64_t i = n / 4 * 4 + t0; i < n; i += stride) top = max(top, ids[i]);
+  if (top >= limit && n) atomicOr(bad, 2u);
 }
 
 // Zeroes `words` words (read frontier + changed bitmap of one parity).
@@ -535,41 +542,7 @@ __global__ void pad_offsets(OffT *R, uint64_t n_src, uint64_t n_rows) {
     R[i] = last;
 }
 
-// ---- out-CSR transposition helpers -------------------------------------------
-
-template <typename OffT>
-__global__ void k_row_of_edge(const OffT *__restrict__ R, uint64_t n_rows,
-                              uint64_t n_edges, uint32_t *__restrict__ row) {
-  for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n_edges;
-       e += (uint64_t)gridDim.x * blockDim.x) {
-    uint64_t lo = 0, hi = n_rows;  // largest r with R[r] <= e
-    while (hi - lo > 1) {
-      uint64_t mid = (lo + hi) >> 1;
-      if ((uint64_t)R[mid] <= e) lo = mid; else hi = mid;
-    }
-    row[e] = (uint32_t)lo;
-  }
-}
-
-__global__ void k_count_u32(const uint32_t *__restrict__ keys, uint64_t n,
-                            uint32_t *__restrict__ counts) {
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (uint64_t)gridDim.x * blockDim.x)
-    atomicAdd(counts + keys[i], 1u);
-}
-
-template <typename OffT>
-__global__ void k_gather_out(const uint32_t *__restrict__ order,
-                             const uint32_t *__restrict__ row_of_edge,
-                             const uint32_t *__restrict__ E, uint64_t n,
-                             uint32_t *__restrict__ outC, uint32_t *__restrict__ outE) {
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (uint64_t)gridDim.x * blockDim.x) {
-    const uint32_t e = order[i];
-    outC[i] = row_of_edge[e];
-    if (outE) outE[i] = E ? E[e] : 1u;
-  }
-}
+// ---- row offsets of the other width -------------------------------------------
 
 template <typename OffT>
 __global__ void k_widen_offsets(const uint32_t *__restrict__ in, uint64_t n,
