@@ -21,10 +21,11 @@ namespace kites_internal {
 // per SM); eight at three CTAs hold as many rows but fewer warps: R-MAT
 // scale 24, K = 64, learned + batched 306.0 against 288.8 GTEPS.
 constexpr int kAsyncRows = 6;
+constexpr int kAsyncBytes = kAsyncRows * 32;   // a lane's copies in flight
 
 // Dynamic shared memory per CTA: per warp, per row slot, 32 bytes per lane.
 constexpr size_t async_batch_smem_bytes() {
-  return (size_t)kWarpsPerBlock * kAsyncRows * 32 * 32;
+  return (size_t)kWarpsPerBlock * 32 * kAsyncBytes;
 }
 
 __device__ __forceinline__ void cp_async_row8(uint4 *smem, const uint32_t *gmem) {
@@ -36,6 +37,11 @@ __device__ __forceinline__ void cp_async_row8(uint4 *smem, const uint32_t *gmem)
       : "memory");
 }
 
+__device__ __forceinline__ void cp_async_16(uint4 *smem, const uint32_t *gmem) {
+  const uint32_t s = (uint32_t)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s), "l"(gmem) : "memory");
+}
+
 __device__ __forceinline__ void cp_async_wait_all() {
   asm volatile("cp.async.wait_all;" ::: "memory");
 }
@@ -44,6 +50,155 @@ __device__ __forceinline__ void smem_row8(const uint4 *smem, uint32_t (&x)[8]) {
   const uint4 p = smem[0], q = smem[1];
   x[0] = p.x; x[1] = p.y; x[2] = p.z; x[3] = p.w;
   x[4] = q.x; x[5] = q.y; x[6] = q.z; x[7] = q.w;
+}
+
+// Rows with more in-edges than this in a chunk take the line-wise copies
+// (row_pieces), from K = 64 on (a row is two lines then).  The fixed pull,
+// before -> after: R-MAT of 2^18 vertices K = 64 2.28 -> 1.88 ms, K = 128 3.64 ->
+// 2.73; 2^20 vertices K = 64 6.42 -> 5.07, K = 256 20.2 -> 13.8; 2^22 K = 64 20.1 ->
+// 17.4, K = 256 70.7 -> 53.0 (16 edges a vertex).  What short rows fetch comes
+// mostly from HBM on the graphs that have many, and line-wise copies of it
+// were slower (Erdos-Renyi, 2^20 vertices, K = 64: 14.1 ms for all rows against
+// 12.3); at K = 16 they gained nothing, and in the masked pull and the push,
+// which copy single sectors, they lost up to 17 %.
+constexpr int64_t kLineRow = 64;
+constexpr int kLineK = 64;
+
+template <int OP>
+__device__ __forceinline__ void fold_piece(const uint4 x, uint32_t w, uint32_t *acc) {
+  acc[0] = min(acc[0], nbr_comp<OP>(x.x, w));
+  acc[1] = min(acc[1], nbr_comp<OP>(x.y, w));
+  acc[2] = min(acc[2], nbr_comp<OP>(x.z, w));
+  acc[3] = min(acc[3], nbr_comp<OP>(x.w, w));
+}
+
+// How a warp covers the source rows of a long row: LPE lanes take a row, each
+// two 16-byte pieces of it (kl and kl + LPE), EPW rows at a time.  Together the
+// lanes copy whole 128-byte lines with each instruction, where 32 contiguous
+// bytes a lane make every instruction touch half of each sector and the two of
+// a row touch each line twice.
+template <int K>
+struct row_pieces {
+  static constexpr int kPieces = 2;
+  static constexpr int VPL = 4 * kPieces;   // values per lane
+  static constexpr int LPE = K / VPL;       // lanes per row
+  static constexpr int EPW = 32 / LPE;      // rows per warp step
+  static constexpr uint32_t kLanes = LPE == 32 ? kFull : ((1u << LPE) - 1u);
+
+  static constexpr int kPullRows = kAsyncBytes / (16 * kPieces);   // in flight per lane
+
+  static __device__ __forceinline__ void load(const uint32_t *p, uint32_t (&x)[VPL]) {
+#pragma unroll
+    for (int h = 0; h < kPieces; ++h)
+      asm volatile("ld.global.L1::no_allocate.v4.b32 {%0,%1,%2,%3}, [%4];"
+                   : "=r"(x[4 * h]), "=r"(x[4 * h + 1]), "=r"(x[4 * h + 2]), "=r"(x[4 * h + 3])
+                   : "l"(p + h * 4 * LPE));
+  }
+  // Bits 2i and 2i + 1 of x joined into bit i.
+  static __device__ __forceinline__ uint32_t pairs(uint32_t x) {
+    x = (x | x >> 1) & 0x55555555u;
+    x = (x | x >> 1) & 0x33333333u;
+    x = (x | x >> 2) & 0x0F0F0F0Fu;
+    x = (x | x >> 4) & 0x00FF00FFu;
+    return (x | x >> 8) & 0xFFFFu;
+  }
+  // Sector bits of lane group `sub`'s row from each lane's pieces (a sector's
+  // halves lie in neighbouring lanes); whole warps.
+  static __device__ __forceinline__ uint32_t sectors(const bool (&piece)[kPieces], uint32_t sub) {
+    uint32_t out = 0;
+#pragma unroll
+    for (int h = 0; h < kPieces; ++h)
+      out |= pairs((__ballot_sync(kFull, piece[h]) >> (sub * LPE)) & kLanes) << (h * LPE / 2);
+    return out;
+  }
+};
+
+// Lowers the lane's values of a row to acc (the lanes of a group together): a
+// row wholly in this chunk is stored, whole, where any value fell; one split
+// over chunks merges with atomicMin.
+template <class P>
+__device__ __forceinline__ void lower_row(uint32_t *dv, const uint32_t (&acc)[P::VPL], bool whole,
+                                          uint32_t sub, bool (&upd)[P::kPieces]) {
+  uint32_t cur[P::VPL];
+  P::load(dv, cur);
+  bool any = false;
+#pragma unroll
+  for (int h = 0; h < P::kPieces; ++h) {
+    uint32_t *to = dv + h * 4 * P::LPE;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int x = 4 * h + q;
+      if (acc[x] >= cur[x]) continue;
+      upd[h] |= whole || acc[x] < atomicMin(to + q, acc[x]);
+      cur[x] = acc[x];
+    }
+    any |= upd[h];
+  }
+  if (whole && __any_sync(P::kLanes << (sub * P::LPE), any)) {
+#pragma unroll
+    for (int h = 0; h < P::kPieces; ++h)
+      *reinterpret_cast<uint4 *>(dv + h * 4 * P::LPE) =
+          make_uint4(cur[4 * h], cur[4 * h + 1], cur[4 * h + 2], cur[4 * h + 3]);
+  }
+}
+
+// Folds in-edges [lo, hi) of one row, line-wise, and lowers the row: the
+// sectors that fell.  Whole warps; `slots` is the warp's kAsyncBytes a lane.
+template <int OP, typename OffT, int K>
+__device__ __forceinline__ uint32_t pull_long_row(const pull_batch_args<OffT> &a, uint64_t v,
+                                                  int64_t lo, int64_t hi, bool whole,
+                                                  uint4 *slots) {
+  using S = row_pieces<K>;
+  constexpr int kRows = S::kPullRows, kPieces = S::kPieces;
+  constexpr int kSlot = 32 * kPieces;   // uint4 of a slot: EPW rows
+  const uint32_t lane = lane_id();
+  const uint32_t sub = lane / S::LPE, kl = lane % S::LPE;
+  // Slot r holds the lane groups' rows one after another, each as it lies in
+  // memory: this lane's pieces are my[r * kSlot + h * LPE].
+  uint4 *my = slots + sub * kPieces * S::LPE + kl;
+  uint32_t acc[S::VPL];
+#pragma unroll
+  for (int q = 0; q < S::VPL; ++q) acc[q] = kInf;
+  for (int64_t tile = lo; tile < hi; tile += 32) {
+    const int64_t t = tile + lane;
+    const uint32_t ntile = (uint32_t)min((int64_t)32, hi - tile);
+    uint32_t cC = 0, cE = 0;
+    if (t < hi) {
+      cC = __ldcs(a.g.C + t);
+      if (op_reads_weights<OP>()) cE = __ldcs(a.E + t);
+    }
+    for (uint32_t jj = 0; jj < ntile; jj += S::EPW * kRows) {
+      uint32_t wq[kRows];
+#pragma unroll
+      for (int r = 0; r < kRows; ++r) {
+        const uint32_t j = jj + r * S::EPW + sub;
+        // Every lane takes part in every shuffle (full mask).
+        const uint32_t u = __shfl_sync(kFull, cC, j & 31u);
+        wq[r] = __shfl_sync(kFull, cE, j & 31u);
+        if (j >= ntile) continue;
+        const uint32_t *du = a.D + (uint64_t)u * K + kl * 4;
+#pragma unroll
+        for (int h = 0; h < kPieces; ++h)
+          cp_async_16(my + r * kSlot + h * S::LPE, du + h * 4 * S::LPE);
+      }
+      cp_async_wait_all();
+#pragma unroll
+      for (int r = 0; r < kRows; ++r) {
+        if (jj + r * S::EPW + sub >= ntile) continue;
+#pragma unroll
+        for (int h = 0; h < kPieces; ++h)
+          fold_piece<OP>(my[r * kSlot + h * S::LPE], wq[r], &acc[4 * h]);
+      }
+    }
+  }
+#pragma unroll
+  for (int d = S::LPE; d < 32; d <<= 1) {
+#pragma unroll
+    for (int q = 0; q < S::VPL; ++q) acc[q] = min(acc[q], __shfl_xor_sync(kFull, acc[q], d));
+  }
+  bool upd[kPieces] = {};
+  if (sub == 0) lower_row<S>(a.D + v * K + kl * 4, acc, whole, 0u, upd);
+  return S::sectors(upd, 0u);
 }
 
 template <int OP, typename OffT, int K, bool kMasked = false>
@@ -167,6 +322,17 @@ __global__ void __launch_bounds__(kBlock, 4) k_pull_batch_async(pull_batch_args<
         if (hi <= lo) continue;
         if (lane == 0) n_edges += (uint64_t)(hi - lo);
         const bool whole = lo == r0 && hi == r1;
+        if constexpr (!kMasked && K >= kLineK) {
+          if (hi - lo > kLineRow) {
+            const uint32_t sec = pull_long_row<OP, OffT, K>(
+                a, v, lo, hi, whole, s_rows + (size_t)wib * kAsyncRows * 64);
+            if (sec) {
+              upd_bits |= 1u << b;
+              if (a.Mnext && lane == 0) atomicOr(a.Mnext + v, sec);
+            }
+            continue;
+          }
+        }
         uint32_t acc[S::VPL];
 #pragma unroll
         for (int q = 0; q < S::VPL; ++q) acc[q] = kInf;
