@@ -111,10 +111,10 @@ int set_device(kites_engine *eng) {
 }
 
 template <typename OffT>
-int build_chunk_table(kites_graph *g, const OffT *R, uint64_t n_rows,
-                      uint64_t n_edges, uint32_t **table, uint64_t *nchunks) {
+int build_chunk_table(kites_graph *g, const OffT *R, uint64_t n_rows, uint64_t n_edges,
+                      uint32_t chunk_items, uint32_t **table, uint64_t *nchunks) {
   const uint64_t items = n_rows + n_edges;
-  uint64_t nc = (items + g->chunk_items - 1) / g->chunk_items;
+  uint64_t nc = (items + chunk_items - 1) / chunk_items;
   if (nc == 0) nc = 1;
   void *p;
   KITES_TRY(graph_alloc(g, &p, (nc + 1) * sizeof(uint32_t)));
@@ -125,7 +125,7 @@ int build_chunk_table(kites_graph *g, const OffT *R, uint64_t n_rows,
     return KITES_OK;
   }
   k_chunk_table<OffT><<<grid_for(nc + 1), 256, 0, g->eng->stream>>>(
-      R, n_rows, nc, g->chunk_items, *table);
+      R, n_rows, nc, chunk_items, *table);
   KITES_CUDA_TRY(cudaGetLastError());
   return KITES_OK;
 }
@@ -378,14 +378,21 @@ int upload_typed(kites_graph *g, const kites_csc_view *v, const built_csc *built
     KITES_TRY(validate_csc<OffT>(g, dR, g->n_dir_rows, g->n_dir_edges, g->dirC, ngroups,
                                  "group out-adjacency"));
   }
-  KITES_TRY(build_chunk_table<OffT>(g, (const OffT *)g->R, g->n, g->m, &g->chunk_in,
-                                    &g->nchunks_in));
+  KITES_TRY(build_chunk_table<OffT>(g, (const OffT *)g->R, g->n, g->m, g->chunk_items,
+                                    &g->chunk_in, &g->nchunks_in));
   if (g->dirR == g->R) {
     g->chunk_dir = g->chunk_in;
     g->nchunks_dir = g->nchunks_in;
   } else {
-    KITES_TRY(build_chunk_table<OffT>(g, (const OffT *)g->dirR, g->n_dir_rows,
-                                      g->n_dir_edges, &g->chunk_dir, &g->nchunks_dir));
+    // Chunks of the out-rows: the activation walks a changed row's part of one
+    // with a single warp, so small graphs get smaller ones, about two a resident
+    // warp (R-MAT of 131,071 vertices and 2.1 M edges: the activation of 379
+    // rows took 84 us in 136 CTAs with 2,048 items).
+    const uint64_t warps = 40ull * eng->sm_count;
+    while (g->dir_items > 128 && (g->n_dir_rows + g->n_dir_edges) / g->dir_items < 2 * warps)
+      g->dir_items /= 2;
+    KITES_TRY(build_chunk_table<OffT>(g, (const OffT *)g->dirR, g->n_dir_rows, g->n_dir_edges,
+                                      g->dir_items, &g->chunk_dir, &g->nchunks_dir));
   }
 
   int per_sm = 0;
@@ -439,7 +446,8 @@ void launch_expand(kites_graph *g, const void *aR, const uint32_t *aC, const uin
                    bool dense_by_next_pull = false) {
   cudaStream_t s = g->eng->stream;
   const bool sweep = dense_pull && g->rowid != nullptr;
-  chunk_geom<OffT> ga{(const OffT *)aR, aC, chunks, nchunks, rows, rows + edges, g->chunk_items};
+  chunk_geom<OffT> ga{(const OffT *)aR, aC, chunks, nchunks, rows, rows + edges,
+                      chunks == g->chunk_in ? g->chunk_items : g->dir_items};
   expand_args<OffT> ea{ga, chg, wr, g->ctr, sweep ? 1u : 0u, gate_cur, g->dense_rows};
   k_expand_chunked<OffT><<<g->expand_grid, kBlock, 0, s>>>(ea);
   ++*launches;
@@ -450,6 +458,18 @@ void launch_expand(kites_graph *g, const void *aR, const uint32_t *aC, const uin
     k_activate_sweep<OffT><<<g->sweep_grid, kSweepThreads, 0, s>>>(sa);
     ++*launches;
   }
+}
+
+// Enqueues the end of an iteration: clears the ranges and runs the loop check.
+int launch_end(kites_graph *g, const clear_list &cl, cudaGraphConditionalHandle h,
+               int has_handle, uint64_t *launches) {
+  const uint64_t most = std::max(cl.words[0], std::max(cl.words[1], cl.words[2]));
+  const iter_record rec{g->rec_active, g->rec_edges, KITES_MAX_RECORDED_ITERS};
+  k_end_iteration<<<grid_for(most, 256, 4096), 256, 0, g->eng->stream>>>(cl, g->ctr, rec, h,
+                                                                        has_handle);
+  KITES_CUDA_TRY(cudaGetLastError());
+  ++*launches;
+  return KITES_OK;
 }
 
 // One iteration of the plain strategy: pull, activation, clear, check.
@@ -490,17 +510,10 @@ int launch_iteration(kites_graph *g, int parity, cudaGraphConditionalHandle h,
                       g->frontier[parity ^ 1], 1u, launches, sweep);
   // Clear the read frontier and, with sweeps, the previous changed set;
   // without them this iteration's (adjacent words).
-  if (sweep)
-    k_clear_two<<<grid_for(g->nwords, 256, 4096), 256, 0, s>>>(g->frontier[parity],
-                                                                g->changed[parity ^ 1], g->nwords);
-  else
-    k_clear_words<<<grid_for(2 * g->nwords, 256, 4096), 256, 0, s>>>(g->frontier[parity],
-                                                                      2 * g->nwords);
-  iter_record rec{g->rec_active, g->rec_edges, KITES_MAX_RECORDED_ITERS};
-  k_loop_check<<<1, 1, 0, s>>>(g->ctr, rec, h, has_handle);
-  KITES_CUDA_TRY(cudaGetLastError());
-  *launches += 3;
-  return KITES_OK;
+  const clear_list cl{{g->frontier[parity], sweep ? g->changed[parity ^ 1] : g->changed[parity]},
+                      {g->nwords, g->nwords}};
+  *launches += 1;
+  return launch_end(g, cl, h, has_handle, launches);
 }
 
 // Batched iteration: K-wide pull over the V x K array, vertex-level
@@ -566,18 +579,14 @@ int launch_batch_iteration(kites_graph *g, const batch_state &b, int parity,
   if (time_pull) KITES_CUDA_TRY(cudaEventRecord(g->eng->kev1, s));
   launch_expand<OffT>(g, b.actR, b.actC, b.act_chunks, b.act_nchunks, true, b.act_rows,
                       b.act_edges, chg, wr, 1u, launches);
-  k_clear_words<<<grid_for(2 * b.nwords, 256, 4096), 256, 0, s>>>(rd, 2 * b.nwords);
-  iter_record rec{g->rec_active, g->rec_edges, KITES_MAX_RECORDED_ITERS};
-  k_loop_check<<<1, 1, 0, s>>>(g->ctr, rec, h, has_handle);
-  KITES_CUDA_TRY(cudaGetLastError());
-  *launches += 3;
-  return KITES_OK;
+  *launches += 1;
+  return launch_end(g, clear_list{{rd}, {2 * b.nwords}}, h, has_handle, launches);
 }
 
 // Iterates to the fixed point.  `launch(parity, handle, has_handle,
 // &launches, time_pull)` enqueues one iteration.  Device loop: a CUDA graph
 // whose conditional while node runs two iterations per trip and stops when
-// k_loop_check clears the condition; it is captured once per loop key and
+// the check clears the condition; it is captured once per loop key and
 // reused.  Host loop: one counter read-back per iteration, as
 // compute.cuh:57-128 does; with time_kernels it also times each pull.
 template <class Launch>
@@ -922,8 +931,6 @@ int launch_strategy(kites_graph *g, const flex_state &f, int strategy, int parit
   uint32_t *Ucur = f.U[parity], *Unext = f.U[parity ^ 1];
   chunk_geom<OffT> gin{(const OffT *)g->R, g->C, g->chunk_in, g->nchunks_in,
                        g->n, g->n + g->m, g->chunk_items};
-  chunk_geom<OffT> gdir{(const OffT *)g->dirR, g->dirC, g->chunk_dir, g->nchunks_dir,
-                        g->n_dir_rows, g->n_dir_rows + g->n_dir_edges, g->chunk_items};
   const uint64_t nw = g->nwords;
   auto expand = [&]() {
     // U was marked by the previous iteration: its count is last_changed.
@@ -1012,12 +1019,7 @@ int launch_flex_iteration(kites_graph *g, const flex_state &f, int strategy, int
   if (time_pull) KITES_CUDA_TRY(cudaEventRecord(g->eng->kev0, s));
   KITES_TRY((launch_strategy<OP, OffT>(g, f, strategy, parity, launches)));
   if (time_pull) KITES_CUDA_TRY(cudaEventRecord(g->eng->kev1, s));
-  k_clear_two<<<grid_for(g->nwords, 256, 4096), 256, 0, s>>>(f.A, f.U[parity], g->nwords);
-  iter_record rec{g->rec_active, g->rec_edges, KITES_MAX_RECORDED_ITERS};
-  k_loop_check<<<1, 1, 0, s>>>(g->ctr, rec, h, hh);
-  KITES_CUDA_TRY(cudaGetLastError());
-  *launches += 2;
-  return KITES_OK;
+  return launch_end(g, clear_list{{f.A, f.U[parity]}, {g->nwords, g->nwords}}, h, hh, launches);
 }
 
 // Runs the graph's current values from the changed set in U[0] with one
@@ -1100,11 +1102,11 @@ int launch_select(kites_graph *g, const uint32_t *U, float margin, float *feat_o
                   uint32_t sectors = 0) {
   select_args<OffT> a{U, g->nwords, g->out_deg, (const OffT *)g->R, g->n, g->m, g->ctr,
                       (select_acc *)g->sacc, params ? params : g->eng->sel_params,
-                      logf(1.f + margin), feat_out, feat_cap, h, hh, M, sectors};
+                      logf(1.f + margin), feat_out, feat_cap, h, hh, M, sectors,
+                      g->rec_sel, KITES_MAX_RECORDED_ITERS};
   k_select<OffT><<<grid_for(g->nwords, 256, (unsigned)g->eng->sm_count * 4), 256, 0,
                    g->eng->stream>>>(a);
-  k_record_sel<<<1, 1, 0, g->eng->stream>>>(g->ctr, g->rec_sel, KITES_MAX_RECORDED_ITERS);
-  *launches += 2;
+  ++*launches;
   KITES_CUDA_TRY(cudaGetLastError());
   return KITES_OK;
 }
@@ -1173,11 +1175,7 @@ int build_auto_loop(kites_graph *g, const flex_state &f, float margin, cudaGraph
       }, nullptr));
     }
     KITES_TRY(capture_into(s, body, {snode}, [&]() -> int {
-      k_clear_two<<<grid_for(g->nwords, 256, 4096), 256, 0, s>>>(f.A, f.U[parity], g->nwords);
-      iter_record rec{g->rec_active, g->rec_edges, KITES_MAX_RECORDED_ITERS};
-      k_loop_check<<<1, 1, 0, s>>>(g->ctr, rec, hw, 1);
-      KITES_CUDA_TRY(cudaGetLastError());
-      return KITES_OK;
+      return launch_end(g, clear_list{{f.A, f.U[parity]}, {g->nwords, g->nwords}}, hw, 1, &dummy);
     }, &leaves));
   }
   KITES_CUDA_TRY(cudaGraphInstantiate(exec, graph, 0));
@@ -1484,8 +1482,8 @@ int prepare_batch(kites_graph *g, uint32_t K, uint32_t items, batch_state *b) {
     b->act_nchunks = g->nchunks_dir; b->act_rows = g->n; b->act_edges = g->m;
   } else {
     if (!g->chunk_out)
-      KITES_TRY(build_chunk_table<OffT>(g, (const OffT *)g->outR, g->n, g->m, &g->chunk_out,
-                                        &g->nchunks_out));
+      KITES_TRY(build_chunk_table<OffT>(g, (const OffT *)g->outR, g->n, g->m,
+                                        g->dir_items, &g->chunk_out, &g->nchunks_out));
     b->actR = g->outR; b->actC = g->outC; b->act_chunks = g->chunk_out;
     b->act_nchunks = g->nchunks_out; b->act_rows = g->n; b->act_edges = g->m;
   }
@@ -1702,8 +1700,8 @@ int prepare_batch_flex(kites_graph *g, uint32_t K, batch_flex *f) {
     onc = g->nchunks_dir;
   } else {
     if (!g->chunk_out)
-      KITES_TRY(build_chunk_table<OffT>(g, (const OffT *)g->outR, g->n, g->m, &g->chunk_out,
-                                        &g->nchunks_out));
+      KITES_TRY(build_chunk_table<OffT>(g, (const OffT *)g->outR, g->n, g->m,
+                                        g->dir_items, &g->chunk_out, &g->nchunks_out));
     oc = g->chunk_out;
     onc = g->nchunks_out;
   }
@@ -1799,7 +1797,7 @@ int launch_batch_strategy(kites_graph *g, const batch_flex &f, int strategy, int
     }
     case KITES_STRATEGY_PUSH: {
       chunk_geom<OffT> go{(const OffT *)f.outR, g->outC, f.out_chunks, f.out_nchunks,
-                          g->n, g->n + g->m, g->chunk_items};
+                          g->n, g->n + g->m, g->dir_items};
       push_batch_args<OffT> pa{go, g->outE, f.D, Uc, Mc, Un, Mn, g->ctr};
       if (f.async_push_grid)
         k_push_batch_async<OP, OffT, K>
@@ -1820,14 +1818,8 @@ int launch_batch_strategy(kites_graph *g, const batch_flex &f, int strategy, int
 // M[parity]) and runs the loop check.
 int launch_batch_tail(kites_graph *g, const batch_flex &f, int parity,
                       cudaGraphConditionalHandle h, int hh, uint64_t *launches) {
-  cudaStream_t s = g->eng->stream;
-  k_clear_two<<<grid_for(f.nwords, 256, 4096), 256, 0, s>>>(f.A, f.U[parity], f.nwords);
-  k_clear_words<<<grid_for(g->n, 256, 4096), 256, 0, s>>>(f.M[parity], g->n);
-  iter_record rec{g->rec_active, g->rec_edges, KITES_MAX_RECORDED_ITERS};
-  k_loop_check<<<1, 1, 0, s>>>(g->ctr, rec, h, hh);
-  KITES_CUDA_TRY(cudaGetLastError());
-  *launches += 3;
-  return KITES_OK;
+  return launch_end(g, clear_list{{f.A, f.U[parity], f.M[parity]}, {f.nwords, f.nwords, g->n}}, h,
+                    hh, launches);
 }
 
 template <int OP, typename OffT, int K>
@@ -2637,12 +2629,14 @@ extern "C" int kites_graph_activate(kites_graph *g, const uint32_t *changed, uin
   cudaStream_t s = g->eng->stream;
   if (g->off64) {
     chunk_geom<uint64_t> ga{(const uint64_t *)g->dirR, g->dirC, g->chunk_dir, g->nchunks_dir,
-                            g->n_dir_rows, g->n_dir_rows + g->n_dir_edges, g->chunk_items};
+                            g->n_dir_rows, g->n_dir_rows + g->n_dir_edges,
+                            g->chunk_dir == g->chunk_in ? g->chunk_items : g->dir_items};
     expand_args<uint64_t> ea{ga, changed, frontier, g->ctr_ext, 0u, 0u, 0ull};
     k_expand_chunked<uint64_t><<<g->expand_grid, kBlock, 0, s>>>(ea);
   } else {
     chunk_geom<uint32_t> ga{(const uint32_t *)g->dirR, g->dirC, g->chunk_dir, g->nchunks_dir,
-                            g->n_dir_rows, g->n_dir_rows + g->n_dir_edges, g->chunk_items};
+                            g->n_dir_rows, g->n_dir_rows + g->n_dir_edges,
+                            g->chunk_dir == g->chunk_in ? g->chunk_items : g->dir_items};
     expand_args<uint32_t> ea{ga, changed, frontier, g->ctr_ext, 0u, 0u, 0ull};
     k_expand_chunked<uint32_t><<<g->expand_grid, kBlock, 0, s>>>(ea);
   }

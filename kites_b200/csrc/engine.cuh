@@ -69,6 +69,7 @@ struct kites_graph {
 
   // Edge-balanced chunk tables.
   uint32_t chunk_items = 2048;
+  uint32_t dir_items = 2048;         // of chunk_dir (where it is not chunk_in) and chunk_out
   uint32_t *chunk_in = nullptr;
   uint64_t nchunks_in = 0;
   uint32_t *chunk_dir = nullptr;

@@ -17,10 +17,10 @@
 //   k_expand_chunked  for each changed row of the activation adjacency
 //                     (dir_R/dir_C, or C for undirected graphs) set the
 //                     out-neighbour bits of the write frontier;
-//   memset            clears the read frontier and the changed bitmap
-//                     (compute.cuh:121);
-//   k_loop_check      counts the iteration and ends the loop when no vertex
-//                     changed (compute.cuh:122-128), on the device.
+//   k_end_iteration   clears the read frontier and the changed bitmap
+//                     (compute.cuh:121), counts the iteration and ends the
+//                     loop when no vertex changed (compute.cuh:122-128), on
+//                     the device.
 #pragma once
 #include "common.cuh"
 
@@ -417,8 +417,8 @@ struct iter_record {
   uint32_t capacity;
 };
 
-__global__ void k_loop_check(run_counters *c, iter_record rec,
-                             cudaGraphConditionalHandle handle, int has_handle) {
+__device__ __forceinline__ void loop_check(run_counters *c, const iter_record &rec,
+                                           cudaGraphConditionalHandle handle, int has_handle) {
   if (c->done) {
     if (has_handle) cudaGraphSetConditional(handle, 0);
     return;
@@ -454,6 +454,27 @@ __global__ void k_loop_check(run_counters *c, iter_record rec,
     c->done = 1;
     if (has_handle) cudaGraphSetConditional(handle, 0);
   }
+}
+
+// Words an iteration leaves empty for the ones to come.
+struct clear_list {
+  uint32_t *p[3];
+  uint64_t words[3];
+};
+
+// Ends an iteration: the consumed bitmaps are cleared by all threads, the loop
+// check runs in the first (it touches counters alone, so neither waits for the
+// other).  One launch where a clear or two and a one-thread check were two or
+// three, 2-4 us each.
+__global__ void __launch_bounds__(256)
+    k_end_iteration(clear_list cl, run_counters *c, iter_record rec,
+                    cudaGraphConditionalHandle handle, int has_handle) {
+  const uint64_t t = (uint64_t)blockIdx.x * 256 + threadIdx.x;
+  if (t == 0) loop_check(c, rec, handle, has_handle);
+  const uint64_t stride = (uint64_t)gridDim.x * 256;
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+    for (uint64_t i = t; i < cl.words[k]; i += stride) cl.p[k][i] = 0u;
 }
 
 // ---- initialisation ---------------------------------------------------------
@@ -524,13 +545,6 @@ __global__ void k_validate_ids(const uint32_t *__restrict__ ids, uint64_t n,
   }
   for (uint64_t i = n / 4 * 4 + t0; i < n; i += stride) top = max(top, ids[i]);
   if (top >= limit && n) atomicOr(bad, 2u);
-}
-
-// Zeroes `words` words (read frontier + changed bitmap of one parity).
-__global__ void k_clear_words(uint32_t *p, uint64_t words) {
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < words;
-       i += (uint64_t)gridDim.x * blockDim.x)
-    p[i] = 0u;
 }
 
 // R[n_src+1 .. n_rows] = R[n_src]: empty rows for the 128-padding vertices.

@@ -54,6 +54,8 @@ struct select_args {
   // changed rows' sectors.
   const uint32_t *M;
   uint32_t sectors;
+  uint8_t *rec_sel;          // class of every iteration
+  uint32_t rec_cap;
 };
 
 // x (kFeat, raw) -> out (kClasses): standardise, two ReLU layers, linear.
@@ -216,6 +218,8 @@ __global__ void __launch_bounds__(256) k_select(select_args<OffT> a) {
   }
   if (lane == 0) {
     a.ctr->sel = cls;
+    // The class picked for the coming iteration, read back for stats.
+    if (a.ctr->iterations < a.rec_cap) a.rec_sel[a.ctr->iterations] = (uint8_t)cls;
     if (a.has_handle) cudaGraphSetConditional(a.handle, cls);
   }
 }
@@ -343,12 +347,6 @@ __global__ void k_mlp_adam(float *P, float *G, float *Mm, float *Vv, float lr, f
   const float vh = v / (1.f - powf(b2, (float)step));
   P[i] -= lr * mh / (sqrtf(vh) + eps);
   G[i] = 0.f;
-}
-
-// Keeps the class picked for the coming iteration (read back for stats).
-__global__ void k_record_sel(const run_counters *c, uint8_t *rec, uint32_t cap) {
-  if (threadIdx.x == 0 && blockIdx.x == 0 && !c->done && c->iterations < cap)
-    rec[c->iterations] = (uint8_t)c->sel;
 }
 
 // Neutral selector: zero weights, unit std -- every prediction is 0, so the

@@ -189,13 +189,4 @@ __global__ void __launch_bounds__(kBlock) k_pull_tpv(pull_tpv_args<OffT> a) {
   }
 }
 
-// Clears two word ranges (the frontier scratch and the consumed changed set).
-__global__ void k_clear_two(uint32_t *a, uint32_t *b, uint64_t words) {
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < words;
-       i += (uint64_t)gridDim.x * blockDim.x) {
-    a[i] = 0u;
-    b[i] = 0u;
-  }
-}
-
 }  // namespace kites_internal
