@@ -264,7 +264,8 @@ int kites_sssp(kites_engine *eng, kites_graph *g, int op, uint32_t source,
  * V x K vertex-major array (dist_out[v*K + k]); K is 16, 32, 64, 128 or 256.
  * opts->strategy: PLAIN (the K-wide pull every iteration), or -- for the
  * saturating SSSP and BFS on graphs with vertex_per_group 1 -- AUTO (the
- * batched learned selector), PUSH, PULL_ALL or PULL_CHANGED. */
+ * batched learned selector; with its default weights and margin the fixed pull
+ * while n_edges * k < 2^29), PUSH, PULL_ALL or PULL_CHANGED. */
 int kites_sssp_batch(kites_engine *eng, kites_graph *g, int op,
                      const uint32_t *sources, uint32_t k, uint32_t *dist_out,
                      const kites_run_opts *opts, kites_run_stats *stats);

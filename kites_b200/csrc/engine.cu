@@ -2857,6 +2857,17 @@ static int sssp_batch(kites_engine *eng, kites_graph *g, int op, const uint32_t 
       return fail(KITES_ERR_INVALID, "source %u (slot %u) out of range", host_src[i], i);
   kites_run_opts o = resolve_opts(opts, true);
   if (stats) memset(stats, 0, sizeof(*stats));
+  // The selector's pass and the switch node cost 20-30 us an iteration; below
+  // 2^29 gathered values a sweep no mix wins that back.  The fixed pull against
+  // AUTO with the selector: R-MAT of 131,071 vertices, 2.1 M edges, K = 16 0.41
+  // against 0.61 ms; 20,000 vertices, 300,000 edges, K = 64 0.65 against 1.06;
+  // 2^18 vertices, 2^22 edges, K = 64 1.87 against 2.08; at 2^20 vertices, 2^24
+  // edges, K = 64 (2^30) 5.06 against 4.98, Erdos-Renyi 12.4 against 9.7.
+  if (o.strategy == KITES_STRATEGY_AUTO && g->eng->sel_batch_default &&
+      (!opts || opts->selector_margin < 0.f) && o.device_loop && !o.time_kernels &&
+      !o.record_iterations && (op == OP_SSSP || op == OP_BFS) && g->vpg == 1 && g->outE &&
+      g->m * k < (1ull << 29))
+    o.strategy = KITES_STRATEGY_PLAIN;
   if (o.strategy != KITES_STRATEGY_PLAIN) {
     if (o.strategy != KITES_STRATEGY_AUTO && o.strategy != KITES_STRATEGY_PUSH &&
         o.strategy != KITES_STRATEGY_PULL_ALL && o.strategy != KITES_STRATEGY_PULL_CHANGED)
@@ -3040,6 +3051,7 @@ extern "C" int kites_selector_load_batch(kites_engine *eng, const float *params,
   if (n_params != (uint32_t)kParams)
     return fail(KITES_ERR_INVALID, "selector has %d parameters, got %u", kParams, n_params);
   KITES_TRY(set_device(eng));
+  eng->sel_batch_default = false;
   KITES_CUDA_TRY(cudaMemcpyAsync(eng->sel_params_batch, params, kParams * 4, cudaMemcpyDefault,
                                  eng->stream));
   KITES_CUDA_TRY(cudaStreamSynchronize(eng->stream));

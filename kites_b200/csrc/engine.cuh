@@ -26,6 +26,7 @@ struct kites_engine {
   float *sel_params = nullptr;    // learned selector weights (device), or null
   bool sel_default = true;        // they are the compiled-in ones
   float *sel_params_batch = nullptr;  // the batched loop's selector weights
+  bool sel_batch_default = true;  // they are the compiled-in ones
   std::vector<struct kites_graph *> graphs;   // live graphs, destroyed with the engine
 };
 
