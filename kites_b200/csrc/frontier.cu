@@ -2,6 +2,7 @@
 #include "frontier.cuh"
 
 #include <algorithm>
+#include <mutex>
 
 #include "kernels_frontier.cuh"
 
@@ -16,6 +17,14 @@ size_t frontier_bytes(const kites_graph *g, size_t *queues) {
 }
 
 namespace {
+
+// The grid waits for its own CTAs, one on every SM, so two such kernels must
+// not each hold a part of the chip: engines of other threads wait here.  (The
+// kernel fills the chip; side by side they would only take turns.)
+std::mutex &device_lock(int device) {
+  static std::mutex locks[64];
+  return locks[device & 63];
+}
 
 template <int OP, typename OffT>
 int launch(kites_graph *g, int seed, uint32_t source, frontier_result *out, float *ms) {
@@ -54,6 +63,7 @@ int launch(kites_graph *g, int seed, uint32_t source, frontier_result *out, floa
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const uint64_t want = (g->n + g->m) / kFrItems + 1;
   const unsigned grid = (unsigned)std::min<uint64_t>(want, eng->sm_count);
+  std::lock_guard<std::mutex> hold(device_lock(eng->device));
   KITES_CUDA_TRY(cudaMemsetAsync(a.ctl, 0, sizeof(frontier_ctl), s));
   KITES_CUDA_TRY(cudaEventRecord(eng->ev0, s));
   void *args[] = {&a};

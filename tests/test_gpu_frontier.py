@@ -159,3 +159,34 @@ def test_process_states(engine, op, oop, state):
         np.testing.assert_array_equal(got[0], got[1])
     finally:
         g.close()
+
+
+def test_engines_of_several_threads():
+    """Engines of different threads answer at the same time, each what it
+    answers alone."""
+    import threading
+
+    n = 1 << 13
+    s, d, w = capi.gen_rmat(13, 16 * n, seed=4)
+    R, C, E = capi.csc_from_edges(n, s, d, w)
+    want = {src: oracle(R, C, E, n, [src], O.OP_SSSP_SAT) for src in (1, 77)}
+    bad = []
+
+    def serve(src):
+        eng = capi.Engine(0)
+        try:
+            g = capi.Graph(eng, R, C, E)
+            for _ in range(20):
+                if not np.array_equal(g.sssp(src)[0], want[src]):
+                    bad.append(src)
+        except Exception as e:   # a thread's exception must fail the test
+            bad.append(e)
+        finally:
+            eng.close()
+
+    threads = [threading.Thread(target=serve, args=(src,)) for src in want for _ in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad, bad
