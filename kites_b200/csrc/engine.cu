@@ -843,7 +843,7 @@ int run_pagerank(kites_graph *g, uint64_t n_real, float *out, const kites_run_op
 // AUTO takes it while the selector's weights, margin and coarse class are the
 // defaults: against the selector's mix it ran R-MAT of 2.0 M vertices and 32 M
 // edges in 0.95 against 1.41 ms (SSSP) and an Erdos-Renyi graph of 2^20
-// vertices and 2^24 edges in 0.26 against 0.56 ms (BFS); weights loaded or
+// vertices and 2^24 edges in 0.18 against 0.56 ms (BFS); weights loaded or
 // trained by the caller make per-iteration picks.
 bool frontier_applies(const kites_graph *g, int op, const kites_run_opts &o) {
   if (g->vpg != 1 || !g->directed || g->vsize != 4 || !g->outR || !g->outE) return false;
