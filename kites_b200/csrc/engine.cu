@@ -1431,6 +1431,18 @@ static bool encode_batch_map(kites_graph *g, uint32_t K) {
   return true;
 }
 
+// Items of a chunk of the batched pull: the autotuner's, else 256, halved, to 32
+// at least, while there are fewer than two chunks an SM.  (Erdos-Renyi, 2,003
+// vertices, 5 edges each: K = 256 0.95 -> 0.52 ms, K = 64 0.60 -> 0.50.  More, smaller
+// chunks than that split rows and see less of the sweep's own progress: 10,007
+// vertices, 12 edges each, K = 64 took 0.67 ms with 256 items and 0.90 with 32.)
+uint32_t batch_items(const kites_graph *g) {
+  if (g->batch_items_req) return g->batch_items_req;
+  uint32_t items = 256;
+  while (items > 32 && (g->n + g->m) / items < 2ull * g->eng->sm_count) items /= 2;
+  return items;
+}
+
 template <typename OffT>
 int prepare_batch(kites_graph *g, uint32_t K, uint32_t items, batch_state *b) {
   kites_engine *eng = g->eng;
@@ -1543,7 +1555,7 @@ int run_batch(kites_graph *g, const uint32_t *sources, uint32_t *dist_out,
   cudaStream_t s = eng->stream;
   auto t0 = std::chrono::steady_clock::now();
   batch_state b{};
-  const uint32_t items = g->batch_items_req ? g->batch_items_req : 256u;
+  const uint32_t items = batch_items(g);
   KITES_TRY(prepare_batch<OffT>(g, K, items, &b));
   int per_sm = 0;
   KITES_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
@@ -1684,7 +1696,7 @@ int prepare_batch_flex(kites_graph *g, uint32_t K, batch_flex *f) {
   if (g->vpg != 1)
     return fail(KITES_ERR_UNSUPPORTED, "batched strategies need vertex_per_group 1");
   batch_state b{};
-  const uint32_t items = g->batch_items_req ? g->batch_items_req : 256u;
+  const uint32_t items = batch_items(g);
   KITES_TRY(prepare_batch<OffT>(g, K, items, &b));
   void *p;
   if (!g->bmask) {
@@ -3236,7 +3248,7 @@ extern "C" int kites_autotune(kites_engine *eng, kites_graph *g, int op, const u
     g->batch_items_req = bc;
     out->batch_ms = best;
   }
-  out->batch_chunk_items = g->batch_items_req ? g->batch_items_req : 256u;
+  out->batch_chunk_items = batch_items(g);
   return KITES_OK;
 }
 

@@ -102,7 +102,7 @@ struct kites_graph {
   uint32_t *bbits = nullptr;         // vertex-level [f0|c0|f1|c1] when vpg > 1
   uint64_t bnwords = 0;
   uint32_t batch_chunk_items = 0;    // chunk size chunk_batch was built with
-  uint32_t batch_items_req = 0;      // chunk size asked for (autotuner), 0 = 256
+  uint32_t batch_items_req = 0;      // chunk size asked for (autotuner), 0 = by size
   uint32_t *chunk_batch = nullptr;
   uint64_t nchunks_batch = 0;
   uint32_t *chunk_out = nullptr;     // vertex-level out-CSR chunks (vpg > 1)

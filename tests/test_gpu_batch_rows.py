@@ -34,3 +34,28 @@ def test_row_lengths(engine, deg, k, offsets64):
             np.testing.assert_array_equal(loads[:, j], g.sssp(int(srcs[j]))[0])
     finally:
         g.close()
+
+
+@pytest.mark.parametrize("k", [64, 128])
+@pytest.mark.parametrize("deg", [64, 65, 257, 900])
+def test_long_rows_in_large_chunks(engine, deg, k):
+    """A graph large enough for 256-item chunks, where line-wise rows occur."""
+    import torch
+
+    n = 700001
+    rng = np.random.default_rng(deg + k)
+    rows = rng.choice(n, 40, replace=False).astype(np.uint32)
+    ids = np.arange(n, dtype=np.uint32)   # a tree, three children a vertex
+    s = np.concatenate([ids // 3] + [rng.choice(n, deg, replace=False) for _ in rows]).astype(np.uint32)
+    d = np.concatenate([ids, np.repeat(rows, deg)]).astype(np.uint32)
+    w = rng.integers(1, 1000, s.shape[0], dtype=np.uint32)
+    srcs = np.arange(k, dtype=np.uint32)
+    g = capi.Graph.from_edges(engine, n, s, d, w)
+    try:
+        out = [torch.empty((n, k), dtype=torch.int32, device="cuda") for _ in range(2)]
+        for mode in (0, 2):
+            g.set_batch_gather(mode)
+            g.sssp_batch(srcs, out=out[mode // 2])
+        assert torch.equal(out[0], out[1])
+    finally:
+        g.close()
