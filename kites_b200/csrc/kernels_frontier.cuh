@@ -590,7 +590,10 @@ struct frontier_run {
     const uint32_t segs = __ldcg(&cur()->bticket);
     for (uint32_t i = wib * gridDim.x + blockIdx.x; i < segs; i += gridDim.x * kFrWarps) {
       const uint2 en = __ldcg(a.big[qp] + i);
-      if (__ldcg(a.V + en.x) != kInf) continue;
+      // One lane looks: other CTAs may be lowering the word, and the warp has to
+      // take one way with the votes behind it.
+      const uint32_t now = lane == 0 ? __ldcg(a.V + en.x) : 0u;
+      if (__shfl_sync(kFull, now, 0) != kInf) continue;
       const OffT r = a.R[en.x] + (OffT)kProbe + (OffT)en.y * kLongRow, e = a.R[en.x + 1];
       if (!scan(r, e - r > (OffT)kLongRow ? r + (OffT)kLongRow : e)) continue;
       bool mine = false;

@@ -120,6 +120,34 @@ def test_bottom_up_rows(engine, deg, offsets64):
         g.close()
 
 
+@pytest.mark.parametrize("parents", [1, 1500, 3000])
+def test_bottom_up_rows_reached_from_several_segments(engine, parents):
+    """Rows that several CTAs look through at the same time, each finding a
+    parent: one of them queues the row, and the level below it is right."""
+    n, mids = 60000, np.arange(57000, 60000, dtype=np.uint32)
+    rng = np.random.default_rng(parents)
+    rows = np.arange(30000, 30040, dtype=np.uint32)
+    s = [np.zeros(mids.shape[0], np.uint32), np.repeat(mids, 100)]
+    d = [mids, rng.integers(31000, 57000, 100 * mids.shape[0], dtype=np.uint32)]
+    for row in rows:                        # 2,000 in-neighbours never reached come first
+        s += [rng.choice(np.arange(1, 20000, dtype=np.uint32), 2000, replace=False),
+              rng.choice(mids, parents, replace=False)]
+        d.append(np.full(2000 + parents, row, np.uint32))
+    s.append(rows)
+    d.append(rows + np.uint32(500))
+    s, d = np.concatenate(s), np.concatenate(d)
+    R, C, _ = capi.csc_from_edges(n, s, d)
+    g = capi.Graph(engine, R, C, None)
+    try:
+        want = oracle(R, C, None, n, [0], O.OP_BFS_SAT)
+        for _ in range(5):
+            dist, _ = g.sssp(0, op=capi.OP_BFS)
+            np.testing.assert_array_equal(dist, want)
+        assert (want[rows] == 2).all() and (want[rows + 500] == 3).sum() > 0
+    finally:
+        g.close()
+
+
 @pytest.mark.parametrize("op,oop", OPS + [(capi.OP_CC, None)])
 @pytest.mark.parametrize("state", ["sources", "missing", "partial", "empty", "settled"])
 def test_process_states(engine, op, oop, state):
