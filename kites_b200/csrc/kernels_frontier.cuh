@@ -45,6 +45,7 @@
 #pragma once
 #include "common.cuh"
 #include "frontier.cuh"
+#include "grid_wait.h"
 
 namespace kites_internal {
 
@@ -65,7 +66,6 @@ constexpr uint32_t kFlush = 128;              // queue entries a warp appends to
 constexpr uint32_t kFarFlush = 96;
 constexpr uint32_t kBatchEdges = 1024;        // out-edges of a wide batch, about
 constexpr uint32_t kFrSpins = 1u << 23;       // bound of the barrier's wait (seconds)
-constexpr uint32_t kFrError = 0x80000000u;    // barrier bit: a CTA gave up
 constexpr uint64_t kFrItems = 512;            // vertices + out-edges that earn a CTA
 constexpr uint64_t kSplitEdges = 16u << 20;   // threshold rule, see run()
 constexpr uint32_t kWideLow = 768u << 10, kWideHigh = 4u << 20;
@@ -86,8 +86,8 @@ struct frontier_slot {
 // ring like the slots: a split reads far_n[far_c], leaves its count in the
 // next one and clears the one after that.
 struct frontier_ctl {
-  unsigned int barrier, violated;
-  uint32_t error, pad;
+  grid_word barrier;
+  uint32_t violated, error;
   frontier_slot slot[3];
   uint32_t far_n[3], pad2;
   unsigned long long wsum;             // sampled weights
@@ -120,8 +120,13 @@ __device__ __forceinline__ uint32_t ld_acquire_u32(const uint32_t *p) {
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
-__device__ __forceinline__ void red_release_add(uint32_t *p, uint32_t x) {
-  asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(x) : "memory");
+__device__ __forceinline__ grid_word ld_acquire_u64(const grid_word *p) {
+  grid_word v;
+  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void red_release_add(grid_word *p, grid_word x) {
+  asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(x) : "memory");
 }
 
 // Sum over the warp: one REDUX while the lanes' values are small.
@@ -143,8 +148,8 @@ struct frontier_run {
   frontier_smem &sm;
   const uint32_t lane, wib;
   // Uniform over the grid.
-  uint32_t step = 0;      // slot[step % 3] is consumed, slot[(step + 1) % 3] filled
-  uint32_t met = 0;       // grid barriers passed
+  uint32_t ring = 0;      // slot[ring] is consumed, the one after it filled
+  grid_word met = 0;      // grid barriers passed
   uint32_t qp = 0;        // q[qp], big[qp] are consumed, queued bits parity qp
   uint32_t fc = 0;        // far list in use
   uint32_t far_c = 0;     // its count: ctl->far_n[far_c]
@@ -162,29 +167,31 @@ struct frontier_run {
 
   __device__ uint32_t *queued(uint32_t p) const { return a.bits + (uint64_t)p * a.nwords; }
   __device__ uint32_t *far_bits() const { return a.bits + 2 * a.nwords; }
-  __device__ uint32_t far_next() const { return far_c == 2u ? 0u : far_c + 1u; }
-  __device__ frontier_slot *cur() const { return &a.ctl->slot[step % 3]; }
-  __device__ frontier_slot *next() const { return &a.ctl->slot[(step + 1) % 3]; }
+  static __device__ uint32_t ring_after(uint32_t i) { return i == 2u ? 0u : i + 1u; }
+  __device__ uint32_t far_next() const { return ring_after(far_c); }
+  __device__ frontier_slot *cur() const { return &a.ctl->slot[ring]; }
+  __device__ frontier_slot *next() const { return &a.ctl->slot[ring_after(ring)]; }
 
   // Called by warp 0 after a CTA barrier: arrives and waits for the grid.
   // False when the wait ran out or another CTA gave up.
   __device__ bool meet() {
     ++met;
-    uint32_t seen = 0;
+    bool failed = false;
     if (lane == 0) {
       red_release_add(&a.ctl->barrier, 1u);
-      const uint32_t target = met * gridDim.x;
       uint32_t spins = 0;
-      while ((seen = ld_acquire_u32(&a.ctl->barrier)) < target) {
+      grid_word seen;
+      while (!grid_met(seen = ld_acquire_u64(&a.ctl->barrier), met, gridDim.x)) {
         if (++spins > 64u) __nanosleep(spins > 4096u ? 256 : 32);
         if (spins > kFrSpins) {
           a.ctl->error = kErrWait;
-          seen = atomicOr(&a.ctl->barrier, kFrError) | kFrError;
+          seen = atomicOr(&a.ctl->barrier, kGridGaveUp) | kGridGaveUp;
           break;
         }
       }
+      failed = grid_failed(seen);
     }
-    return !(__shfl_sync(kFull, seen, 0) & kFrError);
+    return !__any_sync(kFull, failed);
   }
 
   // ---- appends (called by whole warps) ------------------------------------
@@ -274,7 +281,7 @@ struct frontier_run {
         if (smin != kInf) atomicMin(&next()->minv, smin);
         if (blockIdx.x == 0) {
           // The slot of the previous step: nobody reads it any more.
-          frontier_slot *old = &a.ctl->slot[(step + 2) % 3];
+          frontier_slot *old = &a.ctl->slot[ring_after(ring_after(ring))];
           old->qn = old->bn = old->ticket = old->bticket = 0;
           old->edges = old->row_edges = 0;
           old->minv = kInf;
@@ -291,7 +298,7 @@ struct frontier_run {
       ++met;
     }
     __syncthreads();
-    ++step;
+    ring = ring_after(ring);
     return s_ok != 0u;
   }
 
