@@ -156,6 +156,9 @@ __device__ __forceinline__ uint32_t pull_long_row(const pull_batch_args<OffT> &a
   // Slot r holds the lane groups' rows one after another, each as it lies in
   // memory: this lane's pieces are my[r * kSlot + h * LPE].
   uint4 *my = slots + sub * kPieces * S::LPE + kl;
+  // The other rows' slots are laid out per lane: what a lane copies here lies
+  // where another has read its own, and the other way round after this row.
+  __syncwarp();
   uint32_t acc[S::VPL];
 #pragma unroll
   for (int q = 0; q < S::VPL; ++q) acc[q] = kInf;
@@ -191,6 +194,7 @@ __device__ __forceinline__ uint32_t pull_long_row(const pull_batch_args<OffT> &a
       }
     }
   }
+  __syncwarp();
 #pragma unroll
   for (int d = S::LPE; d < 32; d <<= 1) {
 #pragma unroll
