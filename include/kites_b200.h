@@ -201,6 +201,12 @@ int kites_engine_mem_usage(kites_engine *eng, uint64_t *used, uint64_t *total,
 /* nv_gpu::sync (nv_gpu.cuh:45-48): waits for the engine stream and for the
  * copies of kites_sssp_batch_async. */
 int kites_engine_sync(kites_engine *eng);
+/* Bounds the wait of a kernel's CTAs for one another (the single-launch loop
+ * behind PLAIN and AUTO runs): a CTA that has looked `polls` times in vain gives
+ * up, and the call ends with KITES_ERR_TIMEOUT and unfinished values; the engine
+ * and the graph stay usable.  0 restores the default, 2^23 looks (some
+ * seconds).  No reference counterpart. */
+int kites_engine_set_wait_limit(kites_engine *eng, uint32_t polls);
 /* Orders the engine stream after every copy kites_sssp_batch_async has
  * issued so far, without blocking the host (no reference counterpart). */
 int kites_engine_join(kites_engine *eng);

@@ -42,7 +42,7 @@ EXPORTED = [
     "kites_selector_fit", "kites_selector_record_batch", "kites_selector_load_batch",
     "kites_selector_save_batch", "kites_graph_activate", "kites_sssp_batch_async",
     "kites_engine_join", "kites_graph_build_mipmap", "kites_graph_get_mipmap",
-    "kites_graph_set_coarse",
+    "kites_graph_set_coarse", "kites_engine_set_wait_limit",
 ]
 # Selector classes of the batched loop (kites_sssp_batch with AUTO).
 BATCH_CLASS_STRATEGY = [STRATEGY_PLAIN, STRATEGY_PUSH, STRATEGY_PULL_ALL, STRATEGY_PULL_CHANGED]
@@ -143,6 +143,7 @@ def load(path: str = LIB_PATH):
         "kites_engine_mem_usage": (c_int, [vp, POINTER(c_uint64), POINTER(c_uint64),
                                            POINTER(c_uint64)]),
         "kites_engine_sync": (c_int, [vp]),
+        "kites_engine_set_wait_limit": (c_int, [vp, u32]),
         "kites_engine_stream": (c_int, [vp, POINTER(c_void_p)]),
         "kites_graph_upload": (c_int, [vp, POINTER(CscView), POINTER(c_void_p)]),
         "kites_graph_destroy": (c_int, [vp]),
@@ -273,6 +274,11 @@ class Engine:
 
     def sync(self):
         _check(load().kites_engine_sync(self._h))
+
+    def set_wait_limit(self, polls):
+        """Looks of a kernel's CTA that waits for the others before the call
+        ends with ERR_TIMEOUT; 0: the default."""
+        _check(load().kites_engine_set_wait_limit(self._h, int(polls)))
 
     # ---- learned selector ----
     def selector_train(self, features, times_ms, epochs=2000, lr=3e-3, seed=1):

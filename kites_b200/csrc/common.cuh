@@ -65,7 +65,9 @@ struct run_counters {
 // run_counters::error bits, set with atomicOr; any bit ends the loop.
 constexpr uint32_t kErrIndex = 1u;    // an index read during the run was out of range
                                       // (the access was skipped)
-constexpr uint32_t kErrWait = 2u;     // a bounded wait on a TMA copy gave up
+constexpr uint32_t kErrWait = 2u;     // a bounded wait gave up: on a TMA copy, or of the
+                                      // frontier loop's CTAs for one another
+constexpr uint32_t kWaitPolls = 1u << 23;   // default bound of that last wait (seconds)
 
 __device__ __forceinline__ void raise_error(run_counters *c, uint32_t bit) {
   atomicOr(&c->error, bit);

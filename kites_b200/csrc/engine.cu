@@ -2335,6 +2335,13 @@ extern "C" int kites_engine_stream(kites_engine *eng, void **stream_out) {
   return KITES_OK;
 }
 
+extern "C" int kites_engine_set_wait_limit(kites_engine *eng, uint32_t polls) {
+  clear_error();
+  if (!eng) return fail(KITES_ERR_INVALID, "null engine");
+  eng->wait_polls = polls ? polls : kWaitPolls;
+  return KITES_OK;
+}
+
 extern "C" int kites_engine_sync(kites_engine *eng) {
   clear_error();
   if (!eng) return fail(KITES_ERR_INVALID, "null engine");

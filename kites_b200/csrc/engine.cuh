@@ -27,6 +27,7 @@ struct kites_engine {
   bool sel_default = true;        // they are the compiled-in ones
   float *sel_params_batch = nullptr;  // the batched loop's selector weights
   bool sel_batch_default = true;  // they are the compiled-in ones
+  uint32_t wait_polls = kites_internal::kWaitPolls;   // looks of a CTA that waits for the others
   std::vector<struct kites_graph *> graphs;   // live graphs, destroyed with the engine
 };
 

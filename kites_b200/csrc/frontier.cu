@@ -53,6 +53,7 @@ int launch(kites_graph *g, int seed, uint32_t source, frontier_result *out, floa
   a.frontier = g->bitmaps;
   a.source = source;
   a.seed = seed;
+  a.polls = eng->wait_polls;
   a.ctl = (frontier_ctl *)g->fr_mem;
   // The kernel writes its result to the engine's pinned scratch, behind the
   // run counters other loops read back there.

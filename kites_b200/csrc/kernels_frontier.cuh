@@ -65,7 +65,6 @@ constexpr uint32_t kCandRoom = 32 * (kWideCand + kWideFlight);
 constexpr uint32_t kFlush = 128;              // queue entries a warp appends together
 constexpr uint32_t kFarFlush = 96;
 constexpr uint32_t kBatchEdges = 1024;        // out-edges of a wide batch, about
-constexpr uint32_t kFrSpins = 1u << 23;       // bound of the barrier's wait (seconds)
 constexpr uint64_t kFrItems = 512;            // vertices + out-edges that earn a CTA
 constexpr uint64_t kSplitEdges = 16u << 20;   // threshold rule, see run()
 constexpr uint32_t kWideLow = 768u << 10, kWideHigh = 4u << 20;
@@ -87,7 +86,7 @@ struct frontier_slot {
 // next one and clears the one after that.
 struct frontier_ctl {
   grid_word barrier;
-  uint32_t violated, error;
+  uint32_t violated, pad;
   frontier_slot slot[3];
   uint32_t far_n[3], pad2;
   unsigned long long wsum;             // sampled weights
@@ -111,6 +110,7 @@ struct frontier_args {
                           // nwords are the caller's frontier)
   uint32_t source;
   int seed;
+  uint32_t polls;         // looks at the barrier before a CTA gives up
   frontier_ctl *ctl;
   frontier_result *out;
 };
@@ -183,8 +183,7 @@ struct frontier_run {
       grid_word seen;
       while (!grid_met(seen = ld_acquire_u64(&a.ctl->barrier), met, gridDim.x)) {
         if (++spins > 64u) __nanosleep(spins > 4096u ? 256 : 32);
-        if (spins > kFrSpins) {
-          a.ctl->error = kErrWait;
+        if (spins > a.polls) {
           seen = atomicOr(&a.ctl->barrier, kGridGaveUp) | kGridGaveUp;
           break;
         }
@@ -736,14 +735,16 @@ struct frontier_run {
       if (sz) atomicAdd(&a.ctl->updated, sz);
     }
     __syncwarp();
-    if (!gave_up) meet();
+    // A CTA that gave up left its flag in the barrier's word, where every later
+    // meeting finds it, so CTA 0 needs no word of its own to tell the host.
+    if (!gave_up) gave_up = !meet();
     if (blockIdx.x == 0 && lane == 0) {
       a.out->iterations = rounds;
       a.out->active = __ldcg(&a.ctl->active);
       a.out->relaxed = __ldcg(&a.ctl->relaxed);
       a.out->updated = __ldcg(&a.ctl->updated);
       a.out->violated = violated ? 1u : 0u;
-      a.out->error = ld_acquire_u32(&a.ctl->error);
+      a.out->error = gave_up ? kErrWait : 0u;
     }
   }
 

@@ -189,6 +189,38 @@ def test_process_states(engine, op, oop, state):
         g.close()
 
 
+def test_wait_limit():
+    """A grid whose CTAs stop waiting for one another ends with an error status,
+    and the next call answers as before."""
+    n = 1 << 15
+    s, d, w = capi.gen_rmat(15, 16 * n, seed=8)
+    seeds = np.array([5, 9], np.uint32)
+    bits = np.full(n // 32, 0xFFFFFFFF, np.uint32)
+    eng = capi.Engine(0)
+    try:
+        g = capi.Graph.from_edges(eng, n, s, d, w)
+
+        def settle():
+            V = np.full(n, INF, np.uint32)
+            V[int(s[1])] = 0
+            g.set_values(V)
+            g.set_frontier(bits, n)
+            g.process(capi.OP_SSSP)
+
+        calls = [lambda: g.sssp(int(s[1])), lambda: g.sssp(int(s[1]), op=capi.OP_BFS), g.cc,
+                 lambda: g.sssp_multi_seed(seeds), settle]
+        want = g.sssp(int(s[1]))[0]
+        for call in calls:
+            eng.set_wait_limit(1)
+            with pytest.raises(capi.KitesError) as e:
+                call()
+            assert e.value.status == capi.ERR_TIMEOUT
+            eng.set_wait_limit(0)
+            np.testing.assert_array_equal(g.sssp(int(s[1]))[0], want)
+    finally:
+        eng.close()
+
+
 def test_engines_of_several_threads():
     """Engines of different threads answer at the same time, each what it
     answers alone."""
