@@ -434,7 +434,7 @@ def run_ours(args):
         g.build_mipmap(args.mip_block)
         if args.coarse == "mip":
             g.set_coarse(capi.STRATEGY_MIP)
-    stream = torch.cuda.ExternalStream(g.device_view().stream, device=device)
+    stream = torch.cuda.ExternalStream(eng.stream(), device=device)
     srcs = pick_sources(outdeg, args.sources, args.seed, offset=rank)
     K = args.batch
     if args.mode == "batch" and args.sources % K:

@@ -115,7 +115,11 @@ typedef struct kites_csc_view {
 } kites_csc_view;
 
 /* Device pointers of an uploaded graph, for the header-side generic kernels
- * (the C++ front-end instantiates user lambdas in the caller's TU). */
+ * (the C++ front-end instantiates user lambdas in the caller's TU).  V, the
+ * frontier and E may be written between calls; the structure stays as it was
+ * uploaded.  PLAIN runs take the weights E holds when they start; PUSH, and
+ * AUTO where its selector picks it, push with those of the last PLAIN SSSP that
+ * went through the single-launch loop, or of the upload. */
 typedef struct kites_device_view {
   uint64_t n_vertices;              /* padded */
   uint64_t n_edges;

@@ -275,6 +275,12 @@ class Engine:
     def sync(self):
         _check(load().kites_engine_sync(self._h))
 
+    def stream(self):
+        """The engine's cudaStream_t (kites_engine_stream)."""
+        out = c_void_p()
+        _check(load().kites_engine_stream(self._h, ctypes.byref(out)))
+        return out.value
+
     def set_wait_limit(self, polls):
         """Looks of a kernel's CTA that waits for the others before the call
         ends with ERR_TIMEOUT; 0: the default."""
@@ -377,8 +383,7 @@ class Graph:
         self._keep = None
         self.n_vertices = int(v.n_vertices)
         self.n_edges = int(v.n_edges)
-        dv = self.device_view()
-        self.n_padded = int(dv.n_vertices)
+        self.n_padded = (self.n_vertices + 127) // 128 * 128
 
     @classmethod
     def from_edges(cls, engine: Engine, n_vertices, src, dst, w=None, directed=True):
@@ -401,7 +406,7 @@ class Graph:
         engine._graphs.add(self)
         self.n_vertices = int(n_vertices)
         self.n_edges = m
-        self.n_padded = int(self.device_view().n_vertices)
+        self.n_padded = (self.n_vertices + 127) // 128 * 128
         return self
 
     def close(self):

@@ -270,6 +270,8 @@ int build_out_csr(kites_graph *g, const uint32_t *row) {
   g->outE = (uint32_t *)p;
   KITES_TRY(graph_alloc(g, &p, (n + 1) * sizeof(uint32_t)));
   g->out_deg = (uint32_t *)p;
+  KITES_TRY(graph_alloc(g, &p, 16));
+  g->e_sum = (unsigned long long *)p;
   // Row ends are 32-bit edge numbers.
   if (m > 0xFFFFFFFFull)
     return fail(KITES_ERR_UNSUPPORTED, "out-CSR build supports < 2^32 edges");
@@ -287,6 +289,63 @@ int build_out_csr(kites_graph *g, const uint32_t *row) {
   }
   KITES_TRY(scan_row_ends<OffT>(eng, ends, ends + n + 1, n, (OffT *)g->outR, g->out_deg));
   KITES_CUDA_TRY(cudaFreeAsync(ends, s));
+  return KITES_OK;
+}
+
+int sum_weights(kites_graph *g, unsigned long long *sum) {
+  cudaStream_t s = g->eng->stream;
+  KITES_CUDA_TRY(cudaMemsetAsync(sum, 0, 8, s));
+  k_weight_sum<<<grid_for(g->m / 4 + 1, 256, 2048), 256, 0, s>>>((const uint32_t *)g->E, g->m, sum);
+  KITES_CUDA_TRY(cudaGetLastError());
+  return KITES_OK;
+}
+
+// Called when pointers of the graph leave the library: the weights may change
+// in place from now on, and outE holds a copy of them in another order.
+// Nothing may be enqueued while the stream is being captured; the copy then
+// counts as out of date.
+void note_view(kites_graph *g) {
+  if (g->viewed) return;
+  g->viewed = true;
+  if (g->esize != 4 || !g->m || !g->outE || set_device(g->eng) != KITES_OK) return;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusActive;
+  if (cudaStreamIsCapturing(g->eng->stream, &cap) != cudaSuccess ||
+      cap != cudaStreamCaptureStatusNone)
+    return;
+  g->e_sum_known = sum_weights(g, g->e_sum) == KITES_OK;
+}
+
+// Brings outE in line with E if E has changed since outE was made: a stream of
+// E and one round trip a call, and one sort by source where it has.
+int refresh_weights(kites_graph *g) {
+  if (!g->viewed || g->esize != 4 || !g->m) return KITES_OK;
+  kites_engine *eng = g->eng;
+  cudaStream_t s = eng->stream;
+  KITES_TRY(sum_weights(g, g->e_sum + 1));
+  unsigned long long *h = (unsigned long long *)((char *)eng->pinned + 3072);
+  KITES_CUDA_TRY(cudaMemcpyAsync(h, g->e_sum, 16, cudaMemcpyDeviceToHost, s));
+  KITES_CUDA_TRY(cudaStreamSynchronize(s));
+  if (g->e_sum_known && h[0] == h[1]) return KITES_OK;
+  void *keys, *temp;
+  size_t temp_bytes = 0;
+  const int bits = bits_for(g->n);
+  KITES_TRY(dev_alloc(eng, &keys, g->m * 4));
+  auto sort = [&](void *t) {
+    return cub::DeviceRadixSort::SortPairs(t, temp_bytes, g->C, (uint32_t *)keys,
+                                           (const uint32_t *)g->E, g->outE, (uint64_t)g->m, 0,
+                                           bits, s);
+  };
+  cudaError_t e = sort(nullptr);
+  int st = e == cudaSuccess ? dev_alloc(eng, &temp, temp_bytes) : KITES_OK;
+  if (e == cudaSuccess && st == KITES_OK) {
+    e = sort(temp);
+    cudaFreeAsync(temp, s);
+  }
+  cudaFreeAsync(keys, s);
+  KITES_TRY(st);
+  KITES_CUDA_TRY(e);
+  KITES_CUDA_TRY(cudaMemcpyAsync(g->e_sum, g->e_sum + 1, 8, cudaMemcpyDeviceToDevice, s));
+  g->e_sum_known = true;
   return KITES_OK;
 }
 
@@ -882,13 +941,18 @@ int run_frontier(kites_graph *g, int op, int seed, uint32_t source, kites_run_st
   return KITES_OK;
 }
 
-// Whether this call runs as the frontier loop, with its buffers in place.  A
-// graph whose queues do not fit in memory goes to the per-iteration loop.
+// Whether this call runs as the frontier loop, with its buffers in place and
+// its weights up to date.  A graph for which there is no memory for either goes
+// to the per-iteration loop (which reads the weights in E).
 bool frontier_ready(kites_graph *g, int op, const kites_run_opts *opts) {
   kites_run_opts o;
   kites_default_run_opts(&o);
   if (opts) o = *opts;
   if (!frontier_applies(g, op, o)) return false;
+  if (op == OP_SSSP && refresh_weights(g) != KITES_OK) {
+    clear_error();
+    return false;
+  }
   if (g->fr_mem) return true;
   size_t queues;
   if (graph_alloc(g, &g->fr_mem, frontier_bytes(g, &queues)) == KITES_OK) return true;
@@ -2617,6 +2681,7 @@ extern "C" int kites_graph_from_edges(kites_engine *eng, uint64_t n_vertices, ui
 extern "C" int kites_graph_device_view(kites_graph *g, kites_device_view *o) {
   clear_error();
   if (!g || !o) return fail(KITES_ERR_INVALID, "null argument");
+  note_view(g);
   o->n_vertices = g->n;
   o->n_edges = g->m;
   o->nbits = g->nbits;

@@ -138,6 +138,12 @@ struct kites_graph {
   float *pr_x = nullptr;         // x twice, split rows' sums, 1 / out-degree: n each
   uint32_t *pr_rowid = nullptr;  // row of every in-edge where there is no rowid
 
+  // Weights a caller may change in place: once a device view has been handed
+  // out, sums over E as outE was made from it and as it is now.
+  bool viewed = false;
+  bool e_sum_known = false;          // e_sum[0] stands for outE
+  unsigned long long *e_sum = nullptr;
+
   void *fr_mem = nullptr;            // k_frontier_run's buffers (allocated on first use)
   bool density_set = false;          // kites_graph_set_density was called
   bool tuning = false;               // kites_autotune is timing the per-iteration loops

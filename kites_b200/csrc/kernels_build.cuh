@@ -155,6 +155,28 @@ __global__ void __launch_bounds__(256)
     if (i0 + k < m) out[i0 + k] = (uint64_t)row[i0 + k] << 32 | E[i0 + k];
 }
 
+// Adds a 64-bit mix of every edge's number and weight to *sum, so that a weight
+// changed in place shows.  A stream of 4 bytes an edge.
+__global__ void __launch_bounds__(256)
+    k_weight_sum(const uint32_t *__restrict__ E, uint64_t m, unsigned long long *sum) {
+  unsigned long long x = 0;
+  const uint64_t stride = (uint64_t)gridDim.x * 256;
+  auto mix = [](uint64_t e, uint32_t w) {   // SplitMix64's finaliser (Steele et al. 2014)
+    uint64_t z = (e << 32 ^ e >> 32) + w + 0x9E3779B97F4A7C15ull;
+    z = (z ^ z >> 30) * 0xBF58476D1CE4E5B9ull;
+    z = (z ^ z >> 27) * 0x94D049BB133111EBull;
+    return z ^ z >> 31;
+  };
+  const uint64_t t = (uint64_t)blockIdx.x * 256 + threadIdx.x;
+  for (uint64_t i = t; i < m / 4; i += stride) {
+    const uint4 w = __ldcs(reinterpret_cast<const uint4 *>(E) + i);
+    x += mix(4 * i, w.x) + mix(4 * i + 1, w.y) + mix(4 * i + 2, w.z) + mix(4 * i + 3, w.w);
+  }
+  for (uint64_t e = m / 4 * 4 + t; e < m; e += stride) x += mix(e, E[e]);
+  x = warp_sum_u64(x);
+  if (lane_id() == 0 && x) atomicAdd(sum, x);
+}
+
 // Edges sorted by source -> outC, outE (PayT: row << 32 | weight, or the row
 // alone and weights of 1) and the sources' row ends.
 template <typename PayT>

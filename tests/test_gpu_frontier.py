@@ -189,6 +189,51 @@ def test_process_states(engine, op, oop, state):
         g.close()
 
 
+@pytest.mark.parametrize("m", [1, 7, 20000, 20003])
+def test_weights_changed_in_place(engine, m):
+    """Runs take the weights that E holds, also those written through the
+    device view after the upload, whichever edge they belong to."""
+    import torch
+
+    class Words:   # device memory as torch sees it
+        def __init__(self, ptr, count):
+            self.__cuda_array_interface__ = {"shape": (count,), "typestr": "<i4",
+                                             "data": (ptr, False), "version": 3}
+
+    n = 3001
+    rng = np.random.default_rng(m)
+    s = rng.integers(0, n, m, dtype=np.uint32)
+    d = rng.integers(0, n, m, dtype=np.uint32)
+    R, C, E = capi.csc_from_edges(n, s, d, rng.integers(1, 100, m, dtype=np.uint32))
+    src = int(C[0])
+    g = capi.Graph(engine, R, C, E)
+    try:
+        dE = torch.as_tensor(Words(g.device_view().E, m), device="cuda")
+        bits = np.zeros(g.n_padded // 32, np.uint32)
+        for change in ([], [0], [m - 1], [m // 2, m // 3], list(range(m)), []):
+            for e in change:
+                E[e] = rng.integers(1, 2**32, dtype=np.uint64)
+            dE.copy_(torch.from_numpy(E.view(np.int32)))
+            torch.cuda.synchronize()
+            want = oracle(R, C, E, n, [src], O.OP_SSSP_SAT)
+            for strategy in (capi.STRATEGY_PLAIN, capi.STRATEGY_AUTO):
+                dist, _ = g.sssp(src, opts=capi.default_opts(strategy=strategy))
+                np.testing.assert_array_equal(dist, want)
+            np.testing.assert_array_equal(g.sssp_multi_seed(np.array([src], np.uint32))[0], want)
+            V = np.full(n, INF, np.uint32)
+            V[src] = 0
+            hop = C == src
+            row = np.repeat(np.arange(n), np.diff(R.astype(np.int64)))
+            bits[:] = 0
+            np.bitwise_or.at(bits, row[hop] >> 5, (1 << (row[hop] & 31)).astype(np.uint32))
+            g.set_values(V)
+            g.set_frontier(bits, n)
+            g.process(capi.OP_SSSP)
+            np.testing.assert_array_equal(g.get_values(n), want)
+    finally:
+        g.close()
+
+
 def test_wait_limit():
     """A grid whose CTAs stop waiting for one another ends with an error status,
     and the next call answers as before."""
