@@ -2531,12 +2531,14 @@ static int upload_graph(kites_engine *eng, const kites_csc_view *v, const built_
 
 // ---- device-side ingestion (edge list -> CSC) -----------------------------
 
-// An array the caller gave, as device memory: itself, or a copy in *tmp.
+// An array the caller gave, as device memory: itself, or a copy in *tmp.  A copy
+// may start at any byte, a kernel's reads at a whole element only.
 static int on_device(kites_engine *eng, const uint32_t *p, uint64_t m, const uint32_t **out,
                      std::vector<void *> *tmp) {
   cudaPointerAttributes attr;
   const bool dev = cudaPointerGetAttributes(&attr, p) == cudaSuccess &&
-                   attr.type == cudaMemoryTypeDevice && attr.device == eng->device;
+                   attr.type == cudaMemoryTypeDevice && attr.device == eng->device &&
+                   (uintptr_t)p % sizeof(uint32_t) == 0;
   cudaGetLastError();
   if (dev) {
     *out = p;

@@ -70,3 +70,32 @@ def test_uploads(engine, n, m, offsets64):
         check(g, n, R, C, E)
     finally:
         g.close()
+
+
+@pytest.mark.parametrize("offset", [1, 2, 3])
+def test_edge_lists_at_any_byte(engine, offset):
+    """Device arrays that start inside an element are copied, as host arrays
+    are."""
+    import ctypes
+
+    import torch
+
+    n, m = 3000, 20001
+    rng = np.random.default_rng(offset)
+    s, d, w = (rng.integers(0, n, m, dtype=np.uint32) for _ in range(3))
+    R, C, E = capi.csc_from_edges(n, s, d, w)
+    keep = []
+    for x in (s, d, w):
+        t = torch.zeros(4 * m + 16, dtype=torch.uint8, device="cuda")
+        t[offset:offset + 4 * m] = torch.from_numpy(x.view(np.uint8)).cuda()
+        keep.append(t)
+    torch.cuda.synchronize()
+    g = capi.Graph.__new__(capi.Graph)
+    g.engine, g._h = engine, ctypes.c_void_p()
+    ptrs = [ctypes.c_void_p(t.data_ptr() + offset) for t in keep]
+    assert capi.load().kites_graph_from_edges(engine._h, n, m, *ptrs, 1,
+                                              ctypes.byref(g._h)) == capi.OK
+    try:
+        check(g, n, R, C, E)
+    finally:
+        g.close()
