@@ -207,49 +207,100 @@ int bits_for(uint64_t n) {
   return b;
 }
 
+// Scratch of one call, given back to the pool when it ends, however it ends.
+struct scratch {
+  kites_engine *eng;
+  std::vector<void *> held;
+  explicit scratch(kites_engine *e) : eng(e) {}
+  scratch(const scratch &) = delete;
+  ~scratch() {
+    for (void *p : held) cudaFreeAsync(p, eng->stream);
+  }
+  template <class T>
+  int get(T **out, size_t bytes) {
+    void *p = nullptr;
+    KITES_TRY(dev_alloc(eng, &p, bytes));
+    held.push_back(p);
+    *out = (T *)p;
+    return KITES_OK;
+  }
+  void drop(void *p) {
+    cudaFreeAsync(p, eng->stream);
+    held.erase(std::remove(held.begin(), held.end(), p), held.end());
+  }
+};
+
 // Offsets [n + 1] from the rows' ends (as mark_ends leaves them, n + 1 zeroed
 // entries each), and the row lengths into deg if it is not null.
 template <typename OffT>
 int scan_row_ends(kites_engine *eng, const uint32_t *first, const uint32_t *last, uint64_t n,
                   OffT *R, uint32_t *deg) {
   cudaStream_t s = eng->stream;
-  void *wide, *temp;
-  KITES_TRY(dev_alloc(eng, &wide, (n + 1) * sizeof(OffT)));
-  k_row_lengths<OffT><<<grid_for(n + 1), 256, 0, s>>>(first, last, n + 1, (OffT *)wide, deg);
+  scratch tmp(eng);
+  OffT *wide;
+  void *temp;
+  KITES_TRY(tmp.get(&wide, (n + 1) * sizeof(OffT)));
+  k_row_lengths<OffT><<<grid_for(n + 1), 256, 0, s>>>(first, last, n + 1, wide, deg);
   size_t temp_bytes = 0;
-  KITES_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, temp_bytes, (OffT *)wide, R,
-                                               (uint64_t)(n + 1), s));
-  KITES_TRY(dev_alloc(eng, &temp, temp_bytes));
-  KITES_CUDA_TRY(cub::DeviceScan::ExclusiveSum(temp, temp_bytes, (OffT *)wide, R,
-                                               (uint64_t)(n + 1), s));
-  KITES_CUDA_TRY(cudaFreeAsync(temp, s));
-  KITES_CUDA_TRY(cudaFreeAsync(wide, s));
+  KITES_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, temp_bytes, wide, R, (uint64_t)(n + 1), s));
+  KITES_TRY(tmp.get(&temp, temp_bytes));
+  KITES_CUDA_TRY(cub::DeviceScan::ExclusiveSum(temp, temp_bytes, wide, R, (uint64_t)(n + 1), s));
   return KITES_OK;
 }
 
-// Sorts (source, payload) pairs of the CSC by source, stably, and unpacks them
-// into outC, outE and the sources' row ends.
+// Sorts the edges by source, stably, and unpacks them into outC, outE and the
+// sources' row ends.  Bytes an edge at the most, with the graph's own arrays
+// (C, E, the rows): weighted 36 while the sort runs -- its keys and payload
+// twice, between which the passes go to and fro, so that CUB needs no second
+// pair of its own (12 more) and outC and outE can wait for the sort's end --,
+// unweighted 24.
 template <typename PayT>
-int transpose_edges(kites_graph *g, const PayT *pay, uint32_t *ends) {
+int transpose_edges(kites_graph *g, const uint32_t *row, uint32_t *ends) {
   kites_engine *eng = g->eng;
   cudaStream_t s = eng->stream;
   const uint64_t n = g->n, m = g->m;
-  void *keys, *pays, *temp;
-  KITES_TRY(dev_alloc(eng, &keys, m * 4));
-  KITES_TRY(dev_alloc(eng, &pays, m * sizeof(PayT)));
-  size_t temp_bytes = 0;
   const int bits = bits_for(n);
-  KITES_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, temp_bytes, g->C, (uint32_t *)keys, pay,
-                                                 (PayT *)pays, (uint64_t)m, 0, bits, s));
-  KITES_TRY(dev_alloc(eng, &temp, temp_bytes));
-  KITES_CUDA_TRY(cub::DeviceRadixSort::SortPairs(temp, temp_bytes, g->C, (uint32_t *)keys, pay,
-                                                 (PayT *)pays, (uint64_t)m, 0, bits, s));
-  k_unpack_edges<PayT><<<grid_of_edges(m, kBuildPer), 256, 0, s>>>(
-      (const uint32_t *)keys, (const PayT *)pays, m, g->outC, g->outE, ends, ends + n + 1);
+  const unsigned grid = grid_of_edges(m, kBuildPer);
+  scratch tmp(eng);
+  uint32_t *keys;
+  PayT *pay;
+  void *temp;
+  size_t temp_bytes = 0;
+  KITES_TRY(tmp.get(&keys, m * 4));
+  KITES_TRY(tmp.get(&pay, m * sizeof(PayT)));
+  if constexpr (sizeof(PayT) == 8) {
+    uint32_t *keys2;
+    PayT *pay2;
+    KITES_TRY(tmp.get(&keys2, m * 4));
+    KITES_TRY(tmp.get(&pay2, m * sizeof(PayT)));
+    k_pack_edges<<<grid, 256, 0, s>>>(row, g->C, (const uint32_t *)g->E, m, keys, pay);
+    KITES_CUDA_TRY(cudaGetLastError());
+    cub::DoubleBuffer<uint32_t> dk(keys, keys2);
+    cub::DoubleBuffer<PayT> dp(pay, pay2);
+    KITES_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, temp_bytes, dk, dp, (uint64_t)m, 0,
+                                                   bits, s));
+    KITES_TRY(tmp.get(&temp, temp_bytes));
+    KITES_CUDA_TRY(cub::DeviceRadixSort::SortPairs(temp, temp_bytes, dk, dp, (uint64_t)m, 0, bits,
+                                                   s));
+    keys = dk.Current();
+    pay = dp.Current();
+    tmp.drop(dk.Alternate());
+    tmp.drop(dp.Alternate());
+  } else {
+    KITES_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, temp_bytes, g->C, keys, row, pay,
+                                                   (uint64_t)m, 0, bits, s));
+    KITES_TRY(tmp.get(&temp, temp_bytes));
+    KITES_CUDA_TRY(cub::DeviceRadixSort::SortPairs(temp, temp_bytes, g->C, keys, row, pay,
+                                                   (uint64_t)m, 0, bits, s));
+  }
+  tmp.drop(temp);
+  void *p;
+  KITES_TRY(graph_alloc(g, &p, m * 4));
+  g->outC = (uint32_t *)p;
+  KITES_TRY(graph_alloc(g, &p, m * 4));
+  g->outE = (uint32_t *)p;
+  k_unpack_edges<PayT><<<grid, 256, 0, s>>>(keys, pay, m, g->outC, g->outE, ends, ends + n + 1);
   KITES_CUDA_TRY(cudaGetLastError());
-  KITES_CUDA_TRY(cudaFreeAsync(temp, s));
-  KITES_CUDA_TRY(cudaFreeAsync(pays, s));
-  KITES_CUDA_TRY(cudaFreeAsync(keys, s));
   return KITES_OK;
 }
 
@@ -264,10 +315,6 @@ int build_out_csr(kites_graph *g, const uint32_t *row) {
   void *p;
   KITES_TRY(graph_alloc(g, &p, (n + 1) * sizeof(OffT)));
   g->outR = p;
-  KITES_TRY(graph_alloc(g, &p, m * sizeof(uint32_t)));
-  g->outC = (uint32_t *)p;
-  KITES_TRY(graph_alloc(g, &p, m * sizeof(uint32_t)));
-  g->outE = (uint32_t *)p;
   KITES_TRY(graph_alloc(g, &p, (n + 1) * sizeof(uint32_t)));
   g->out_deg = (uint32_t *)p;
   KITES_TRY(graph_alloc(g, &p, 16));
@@ -275,21 +322,21 @@ int build_out_csr(kites_graph *g, const uint32_t *row) {
   // Row ends are 32-bit edge numbers.
   if (m > 0xFFFFFFFFull)
     return fail(KITES_ERR_UNSUPPORTED, "out-CSR build supports < 2^32 edges");
-  KITES_TRY(dev_alloc(eng, &p, 2 * (n + 1) * sizeof(uint32_t)));
-  uint32_t *ends = (uint32_t *)p;
+  scratch tmp(eng);
+  uint32_t *ends;
+  KITES_TRY(tmp.get(&ends, 2 * (n + 1) * sizeof(uint32_t)));
   KITES_CUDA_TRY(cudaMemsetAsync(ends, 0, 2 * (n + 1) * sizeof(uint32_t), s));
   if (m && g->esize == 4) {
-    KITES_TRY(dev_alloc(eng, &p, m * 8));
-    k_pack_edges<<<grid_of_edges(m, kBuildPer), 256, 0, s>>>(row, (const uint32_t *)g->E, m,
-                                                            (uint64_t *)p);
-    KITES_TRY(transpose_edges<uint64_t>(g, (const uint64_t *)p, ends));
-    KITES_CUDA_TRY(cudaFreeAsync(p, s));
+    KITES_TRY(transpose_edges<uint64_t>(g, row, ends));
   } else if (m) {
     KITES_TRY(transpose_edges<uint32_t>(g, row, ends));
+  } else {
+    KITES_TRY(graph_alloc(g, &p, 0));
+    g->outC = (uint32_t *)p;
+    KITES_TRY(graph_alloc(g, &p, 0));
+    g->outE = (uint32_t *)p;
   }
-  KITES_TRY(scan_row_ends<OffT>(eng, ends, ends + n + 1, n, (OffT *)g->outR, g->out_deg));
-  KITES_CUDA_TRY(cudaFreeAsync(ends, s));
-  return KITES_OK;
+  return scan_row_ends<OffT>(eng, ends, ends + n + 1, n, (OffT *)g->outR, g->out_deg);
 }
 
 int sum_weights(kites_graph *g, unsigned long long *sum) {
@@ -326,24 +373,18 @@ int refresh_weights(kites_graph *g) {
   KITES_CUDA_TRY(cudaMemcpyAsync(h, g->e_sum, 16, cudaMemcpyDeviceToHost, s));
   KITES_CUDA_TRY(cudaStreamSynchronize(s));
   if (g->e_sum_known && h[0] == h[1]) return KITES_OK;
-  void *keys, *temp;
+  scratch tmp(eng);
+  uint32_t *keys;
+  void *temp;
   size_t temp_bytes = 0;
-  const int bits = bits_for(g->n);
-  KITES_TRY(dev_alloc(eng, &keys, g->m * 4));
+  KITES_TRY(tmp.get(&keys, g->m * 4));
   auto sort = [&](void *t) {
-    return cub::DeviceRadixSort::SortPairs(t, temp_bytes, g->C, (uint32_t *)keys,
-                                           (const uint32_t *)g->E, g->outE, (uint64_t)g->m, 0,
-                                           bits, s);
+    return cub::DeviceRadixSort::SortPairs(t, temp_bytes, g->C, keys, (const uint32_t *)g->E,
+                                           g->outE, (uint64_t)g->m, 0, bits_for(g->n), s);
   };
-  cudaError_t e = sort(nullptr);
-  int st = e == cudaSuccess ? dev_alloc(eng, &temp, temp_bytes) : KITES_OK;
-  if (e == cudaSuccess && st == KITES_OK) {
-    e = sort(temp);
-    cudaFreeAsync(temp, s);
-  }
-  cudaFreeAsync(keys, s);
-  KITES_TRY(st);
-  KITES_CUDA_TRY(e);
+  KITES_CUDA_TRY(sort(nullptr));
+  KITES_TRY(tmp.get(&temp, temp_bytes));
+  KITES_CUDA_TRY(sort(temp));
   KITES_CUDA_TRY(cudaMemcpyAsync(g->e_sum, g->e_sum + 1, 8, cudaMemcpyDeviceToDevice, s));
   g->e_sum_known = true;
   return KITES_OK;

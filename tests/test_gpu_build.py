@@ -99,3 +99,23 @@ def test_edge_lists_at_any_byte(engine, offset):
         check(g, n, R, C, E)
     finally:
         g.close()
+
+
+@pytest.mark.parametrize("weighted,per_edge", [(True, 40), (False, 36)])
+def test_upload_memory(weighted, per_edge):
+    """What an upload holds at the most (the pool keeps what it ever held): per
+    edge, the sort by source with 32-bit edge numbers as its payload needed 40
+    bytes with weights and 36 without."""
+    n, m = 1 << 16, 1 << 24
+    rng = np.random.default_rng(1)
+    C = np.sort(rng.integers(0, n, (n, m // n), dtype=np.uint32), axis=1).reshape(-1)
+    R = np.arange(n + 1, dtype=np.uint32) * np.uint32(m // n)
+    E = rng.integers(1, 256, m, dtype=np.uint32) if weighted else None
+    eng = capi.Engine(0)
+    try:
+        g = capi.Graph(eng, R, C, E)
+        pool = eng.mem_usage()[2]
+        assert pool <= per_edge * m + (96 << 20), pool / m
+        check(g, n, R, C, E)
+    finally:
+        eng.close()
