@@ -10,6 +10,7 @@
 #include <algorithm>
 #include <chrono>
 #include <type_traits>
+#include <utility>
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
 
@@ -2782,11 +2783,31 @@ extern "C" int kites_graph_get_values(kites_graph *g, void *dst, uint64_t n) {
   return KITES_OK;
 }
 
+// Whether values from host memory are finite so often, in a sample, that
+// kites_process would find too many edges to walk (it looks for itself; this
+// spares it the launch).
+static bool looks_settled(const kites_graph *g, const void *src, uint64_t n) {
+  if (g->vsize != 4 || g->m <= kGivenEdges || n < 64) return false;
+  cudaPointerAttributes attr;
+  const bool known = cudaPointerGetAttributes(&attr, src) == cudaSuccess;
+  cudaGetLastError();
+  if (!known || (attr.type != cudaMemoryTypeUnregistered && attr.type != cudaMemoryTypeHost))
+    return false;
+  uint64_t finite = 0;
+  for (uint64_t i = 0; i < 64; ++i) {
+    uint32_t x;
+    memcpy(&x, (const char *)src + (i * n / 64) * 4, 4);
+    finite += x != kInf;
+  }
+  return finite * (g->m / 64) > kGivenEdges;
+}
+
 extern "C" int kites_graph_set_values(kites_graph *g, const void *src, uint64_t n) {
   clear_error();
   if (!g || !src) return fail(KITES_ERR_INVALID, "null argument");
   if (n > g->n) return fail(KITES_ERR_INVALID, "too many values");
   KITES_TRY(set_device(g->eng));
+  g->given = !looks_settled(g, src, n);
   KITES_CUDA_TRY(cudaMemcpyAsync(g->V, src, n * g->vsize, cudaMemcpyDefault, g->eng->stream));
   KITES_CUDA_TRY(cudaStreamSynchronize(g->eng->stream));
   return KITES_OK;
@@ -2826,7 +2847,10 @@ extern "C" int kites_process(kites_engine *eng, kites_graph *g, int op,
                              const kites_run_opts *opts, kites_run_stats *stats) {
   clear_error();
   KITES_TRY(check_graph(eng, g));
-  if ((!opts || opts->strategy == KITES_STRATEGY_PLAIN) && frontier_ready(g, op, opts)) {
+  // Values that a run left are settled as a rule, and the frontier then says
+  // where there is anything to do: the per-iteration loop pulls its rows alone.
+  const bool start = std::exchange(g->given, false) || g->m <= kGivenEdges;
+  if (start && (!opts || opts->strategy == KITES_STRATEGY_PLAIN) && frontier_ready(g, op, opts)) {
     const int st = run_frontier(g, op, kSeedFinite, 0, stats);
     if (st != KITES_ERR_UNSUPPORTED) return st;
   }
@@ -2874,6 +2898,7 @@ extern "C" int kites_sssp(kites_engine *eng, kites_graph *g, int op, uint32_t so
                           kites_run_stats *stats) {
   clear_error();
   KITES_TRY(check_graph(eng, g));
+  g->given = false;
   if (op != OP_SSSP && op != OP_SSSP_WRAP && op != OP_BFS)
     return fail(KITES_ERR_INVALID, "kites_sssp takes SSSP, SSSP_WRAP or BFS");
   if (source >= g->n_given) return fail(KITES_ERR_INVALID, "source %u out of range", source);
@@ -2911,6 +2936,7 @@ extern "C" int kites_cc(kites_engine *eng, kites_graph *g, uint32_t *labels_out,
                         const kites_run_opts *opts, kites_run_stats *stats) {
   clear_error();
   KITES_TRY(check_graph(eng, g));
+  g->given = false;
   cudaStream_t s = eng->stream;
   auto t0 = std::chrono::steady_clock::now();
   if (frontier_ready(g, OP_CC, opts)) {
@@ -2937,6 +2963,7 @@ extern "C" int kites_pagerank(kites_engine *eng, kites_graph *g, uint64_t n_real
                               kites_run_stats *stats) {
   clear_error();
   KITES_TRY(check_graph(eng, g));
+  g->given = false;
   if (n_real == 0 || n_real > g->n) return fail(KITES_ERR_INVALID, "bad n_real");
   kites_run_opts o = resolve_opts(opts);
   if (stats) memset(stats, 0, sizeof(*stats));
@@ -3015,6 +3042,7 @@ extern "C" int kites_sssp_multi_seed(kites_engine *eng, kites_graph *g, int op,
                                      kites_run_stats *stats) {
   clear_error();
   KITES_TRY(check_graph(eng, g));
+  g->given = false;
   if (op != OP_SSSP && op != OP_SSSP_WRAP && op != OP_BFS)
     return fail(KITES_ERR_INVALID, "multi-seed runs take SSSP, SSSP_WRAP or BFS");
   if (!seeds || n_seeds == 0) return fail(KITES_ERR_INVALID, "no seeds");
@@ -3062,6 +3090,7 @@ extern "C" int kites_selector_record(kites_engine *eng, kites_graph *g, int op, 
                                      uint32_t *n_records) {
   clear_error();
   KITES_TRY(check_graph(eng, g));
+  g->given = false;
   if (!features || !times_ms || !n_records || capacity == 0)
     return fail(KITES_ERR_INVALID, "null output or zero capacity");
   if (op != OP_SSSP && op != OP_BFS && op != OP_CC)

@@ -145,6 +145,7 @@ struct kites_graph {
   unsigned long long *e_sum = nullptr;
 
   void *fr_mem = nullptr;            // k_frontier_run's buffers (allocated on first use)
+  bool given = true;                 // V holds a start the caller put there, no run's result
   bool density_set = false;          // kites_graph_set_density was called
   bool tuning = false;               // kites_autotune is timing the per-iteration loops
 

@@ -7,12 +7,22 @@ namespace kites_internal {
 
 constexpr uint32_t kSeg = 256;   // out-edges of one queue entry, at most
 
+// A caller's state is taken (kSeedFinite) while its finite vertices have about
+// this many out-edges at the most, by a sample: they are walked twice, for the
+// check and as the first iteration, however few of them the caller's frontier
+// needs.  From settled values with 100 frontier bits a call took 58 us at 0.10 M
+// out-edges, 94 at 1.6 M and 284 at 16.6 M (R-MAT); pulling the frontier's rows
+// takes the per-iteration loop 80 us whatever the size.  A state that the sample
+// in init() finds too large costs a launch and a wait, about 27 us.
+constexpr uint32_t kGivenEdges = 1u << 20;
+
 // How the run starts.
 enum : int {
   kSeedSource = 0,   // V = INF but 0 at `source`
   kSeedFinite = 1,   // the caller's V and frontier: every vertex below INF is
-                     // queued, after a check that the out-edges whose target is
-                     // outside the frontier are already satisfied
+                     // queued, after a check that they are few enough and that
+                     // the out-edges whose target is outside the frontier are
+                     // already satisfied
   kSeedZeros = 2,    // V is set up; the vertices at 0 are queued
   kSeedLabels = 3    // V[v] = v, every vertex queued
 };

@@ -88,7 +88,7 @@ struct frontier_ctl {
   grid_word barrier;
   uint32_t violated, pad;
   frontier_slot slot[3];
-  uint32_t far_n[3], pad2;
+  uint32_t far_n[3], finite;           // finite: in a sample of the caller's values
   unsigned long long wsum;             // sampled weights
   unsigned long long active, relaxed, updated;
 };
@@ -708,6 +708,13 @@ struct frontier_run {
       wt = warp_sum_u64(wt);
       if (lane == 0 && wt) atomicAdd(&a.ctl->wsum, wt);
     }
+    if (a.seed == kSeedFinite && a.m > kGivenEdges && threadIdx.x < 32) {
+      // 32 vertices a CTA, to leave a state with too many finite ones at once.
+      const uint64_t at =
+          ((uint64_t)blockIdx.x * 32 + lane) * a.n / ((uint64_t)gridDim.x * 32);
+      const uint32_t some = __popc(__ballot_sync(kFull, a.V[at] != kInf));
+      if (lane == 0 && some) atomicAdd(&a.ctl->finite, some);
+    }
     if (blockIdx.x == 0 && threadIdx.x < 3) a.ctl->slot[threadIdx.x].minv = kInf;
   }
 
@@ -762,6 +769,9 @@ struct frontier_run {
       delta = d < 1 ? 1u : d > kInf / 2 ? kInf / 2 : (uint32_t)d;
       thr = delta;
     }
+    if (a.seed == kSeedFinite && a.m > kGivenEdges &&
+        __ldcg(&a.ctl->finite) * a.m / (gridDim.x * 32ull) > kGivenEdges)
+      return finish(true, false);
     // Step 1 queues what other runs start from.
     if (a.seed == kSeedZeros) {
       seed_all([&](uint32_t v) { return __ldcg(a.V + v) == 0u; });
@@ -785,6 +795,7 @@ struct frontier_run {
       // does not satisfy must lead into the caller's frontier, else the
       // iteration of process() would not relax it and the host runs that.
       const frontier_slot sl = s_slot;
+      if (sl.edges > 4 * kGivenEdges) return finish(true, false);   // the sample missed
       wide_push<true>(sl);
       if (blockIdx.x == 0 && threadIdx.x == 0) {   // the queues stay, under the next slot
         frontier_slot *c = next();

@@ -189,6 +189,30 @@ def test_process_states(engine, op, oop, state):
         g.close()
 
 
+@pytest.mark.parametrize("again", [False, True])
+def test_process_of_a_settled_state(engine, again):
+    """From settled values, left by a run or set again, a small frontier costs
+    its own in-edges and not a walk over the graph."""
+    n = 1 << 17
+    s, d, w = capi.gen_rmat(17, 16 * n, seed=6)
+    R, _, _ = capi.csc_from_edges(n, s, d, w)
+    g = capi.Graph.from_edges(engine, n, s, d, w)
+    try:
+        for op in (capi.OP_SSSP, capi.OP_BFS):
+            dist, _ = g.sssp(int(s[77]), op=op)
+            if again:
+                g.set_values(dist)
+            rows = np.array([1, 50, 4000, 65537, n - 1])
+            bits = np.zeros(n, np.uint8)
+            bits[rows] = 1
+            g.set_frontier(np.packbits(bits, bitorder="little").view(np.uint32), n)
+            st = g.process(op)
+            assert st.edges_traversed == int((R[rows + 1] - R[rows]).sum())
+            np.testing.assert_array_equal(g.get_values(n), dist)
+    finally:
+        g.close()
+
+
 @pytest.mark.parametrize("m", [1, 7, 20000, 20003])
 def test_weights_changed_in_place(engine, m):
     """Runs take the weights that E holds, also those written through the
