@@ -401,14 +401,16 @@ int kites_graph_get_mipmap(kites_graph *g, uint64_t *dim_out, uint32_t *words,
  * (vertices + edges per warp), the threads-per-vertex width of the
  * selector's TPV class, its coarse class (PULL_ALL or MIP, on graphs with a
  * block map), and the frontier densities at which the plain loop
- * switches its pull and its activation to the staged sweeps. */
+ * switches its pull and its activation to the staged sweeps.  Densities and
+ * TPV width belong to the per-iteration loops and are timed there; the coarse
+ * class is timed by AUTO runs as they will be. */
 typedef struct kites_tune_result {
   uint32_t batch_chunk_items;
   int32_t tpv_strategy;
   uint64_t dense_edges;
   uint64_t dense_rows;
   float batch_ms;          /* best batched run time             */
-  float plain_ms;          /* best plain single-source run time */
+  float plain_ms;          /* best plain single-source run time, per-iteration loop */
   float tpv_ms;            /* best TPV single-source run time   */
   uint32_t trials;
   int32_t coarse_strategy; /* the selector's coarse class: PULL_ALL or MIP */

@@ -3357,10 +3357,12 @@ extern "C" int kites_autotune(kites_engine *eng, kites_graph *g, int op, const u
   }
   out->tpv_strategy = g->tpv_strategy;
   // 3. The selector's coarse class: PULL_ALL or, on a graph with a block
-  // map, the mipmapped frontier, timed as whole AUTO runs; MIP must win by
-  // 2 % to replace PULL_ALL.
+  // map, the mipmapped frontier, timed as whole AUTO runs, as calls with either
+  // setting will run (with PULL_ALL and the default selector, the single-launch
+  // loop); MIP must win by 2 % to replace PULL_ALL.
   if (g->mip && g->vpg == 1 && g->directed) {
     float t_all = 0.f, t_mip = 0.f;
+    g->tuning = false;
     KITES_TRY(kites_graph_set_coarse(g, KITES_STRATEGY_PULL_ALL));
     KITES_TRY(time_single(KITES_STRATEGY_AUTO, &t_all));
     KITES_TRY(kites_graph_set_coarse(g, KITES_STRATEGY_MIP));

@@ -217,3 +217,27 @@ def test_tpv_guard_on_hub_graph(engine):
     finally:
         engine.selector_load(forced_selector(0))
         g.close()
+
+
+def test_autotune_times_auto_as_it_runs(engine):
+    """The coarse class is chosen between AUTO runs as calls get them: with
+    PULL_ALL and the default selector that is the single-launch loop."""
+    n = 1 << 14
+    s, d, w = capi.gen_rmat(14, 16 * n, seed=9)
+    R, C, E = capi.csc_from_edges(n, s, d, w)
+    eng = capi.Engine(0)
+    try:
+        g = capi.Graph(eng, R, C, E)
+        g.build_mipmap(32)
+        srcs = s[[1, 100, 1000, 10000]]
+        r = g.autotune(srcs, batch=0)
+        assert r.coarse_strategy == capi.STRATEGY_PULL_ALL
+        auto = capi.default_opts(strategy=capi.STRATEGY_AUTO)
+        total = 0.0
+        for src in srcs:
+            runs = [g.sssp(int(src), opts=auto)[1] for _ in range(3)]
+            assert all(st.kernel_launches == 1 for st in runs)
+            total += min(st.device_ms for st in runs)
+        assert r.coarse_ms < 2 * total
+    finally:
+        eng.close()
