@@ -3376,9 +3376,11 @@ extern "C" int kites_autotune(kites_engine *eng, kites_graph *g, int op, const u
   if (batch == 16 || batch == 32 || batch == 64 || batch == 128 || batch == 256) {
     std::vector<uint32_t> bs(batch);
     for (uint32_t i = 0; i < batch; ++i) bs[i] = src[i % n_sources];
-    const uint32_t cands[] = {128, 256, 512, 1024, 2048};
+    std::vector<uint32_t> cands = {128, 256, 512, 1024, 2048};
+    g->batch_items_req = 0;
+    if (batch_items(g) < 128) cands.insert(cands.begin(), {32, 64});   // the untuned size is one
     float best = 1e30f;
-    uint32_t bc = g->batch_chunk_items ? g->batch_chunk_items : 256;
+    uint32_t bc = batch_items(g);
     kites_run_opts bo;
     kites_default_run_opts(&bo);
     for (uint32_t c : cands) {

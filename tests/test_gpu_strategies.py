@@ -219,6 +219,21 @@ def test_tpv_guard_on_hub_graph(engine):
         g.close()
 
 
+def test_autotune_knows_the_untuned_chunk_size(engine):
+    """A graph whose batched runs take chunks below 128 items untuned (K = 256:
+    0.5 ms with 32, 1.0 with 256) is not tuned to larger ones."""
+    n = 2003
+    s, d, w = capi.gen_er(n, 5 * n, seed=3)
+    R, C, E = capi.csc_from_edges(n, s, d, w)
+    g = capi.Graph(engine, R, C, E)
+    srcs = np.arange(256, dtype=np.uint32) * 7
+    before, _ = g.sssp_batch(srcs)
+    r = g.autotune(srcs, batch=256)
+    assert r.batch_chunk_items in (32, 64)
+    np.testing.assert_array_equal(g.sssp_batch(srcs)[0], before)
+    g.close()
+
+
 def test_autotune_times_auto_as_it_runs(engine):
     """The coarse class is chosen between AUTO runs as calls get them: with
     PULL_ALL and the default selector that is the single-launch loop."""
