@@ -56,9 +56,11 @@ typedef enum kites_op {
  * PLAIN runs of SSSP, BFS and CC on directed graphs with vertex_per_group 1
  * go through one kernel that relaxes the out-edges of the changed vertices
  * until nothing changes (same fixed point); so do AUTO runs while the
- * selector, its margin and its coarse class are the defaults.  A host-driven
- * loop (device_loop 0), time_kernels, record_iterations, an iteration limit
- * or kites_graph_set_density keep the pull iteration above.
+ * selector and its margin are the defaults, its coarse class is PULL_ALL and
+ * kites_graph_set_tpv has not been called.  A host-driven loop (device_loop
+ * 0), time_kernels, record_iterations, an iteration limit or
+ * kites_graph_set_density keep the pull iteration above; so does kites_process
+ * from settled values (see there).
  * Batched runs (kites_sssp_batch) take PLAIN, AUTO, PUSH, PULL_ALL and
  * PULL_CHANGED; there PUSH and PULL_CHANGED move only the 32-byte sectors of
  * each source row that changed in the previous iteration, and PULL_ALL
@@ -258,7 +260,10 @@ int kites_graph_activate(kites_graph *g, const uint32_t *changed, uint32_t *fron
 /* kites::process<launch::sync>(devGrph, dev, initF, nbrCompF, redF, updF)
  * (kites/device/compute.cuh:29-137) for a built-in operator: iterates the
  * graph's own vertex values from its current frontier to the fixed point,
- * in place, on the device. */
+ * in place, on the device.  The single-launch loop takes values that the caller
+ * set (kites_graph_upload, kites_graph_set_values) while their finite vertices
+ * have no more than about 2^20 out-edges, and any on graphs of up to 2^20
+ * edges; others, as a run leaves them, are iterated from the frontier. */
 int kites_process(kites_engine *eng, kites_graph *g, int op,
                   const kites_run_opts *opts, kites_run_stats *stats);
 
@@ -368,7 +373,8 @@ int kites_selector_record_batch(kites_engine *eng, kites_graph *g, int op,
 int kites_selector_load_batch(kites_engine *eng, const float *params, uint32_t n_params);
 int kites_selector_save_batch(kites_engine *eng, float *params, uint32_t n_params);
 /* Threads-per-vertex width of the selector's TPV class for this graph
- * (KITES_STRATEGY_TPV1/4/8/32). */
+ * (KITES_STRATEGY_TPV1/4/8/32).  AUTO runs of a graph with the width set go
+ * iteration by iteration, as the selector picks. */
 int kites_graph_set_tpv(kites_graph *g, int strategy);
 /* What the selector's coarse class (class 2) runs on this graph:
  * KITES_STRATEGY_PULL_ALL (default) or KITES_STRATEGY_MIP (needs the block

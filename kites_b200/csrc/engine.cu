@@ -941,8 +941,8 @@ int run_pagerank(kites_graph *g, uint64_t n_real, float *out, const kites_run_op
 // and a program whose comp(INF) is INF, and a caller that asks for nothing
 // that only the iteration-by-iteration loop has (host-driven iterations,
 // per-iteration times or records, an iteration limit, densities set by hand).
-// AUTO takes it while the selector's weights, margin and coarse class are the
-// defaults: against the selector's mix it ran R-MAT of 2.0 M vertices and 32 M
+// AUTO takes it while the selector's weights and margin and its classes' coarse
+// strategy and threads per vertex are the defaults: against the selector's mix it ran R-MAT of 2.0 M vertices and 32 M
 // edges in 0.95 against 1.41 ms (SSSP) and an Erdos-Renyi graph of 2^20
 // vertices and 2^24 edges in 0.18 against 0.56 ms (BFS); weights loaded or
 // trained by the caller make per-iteration picks.
@@ -954,7 +954,7 @@ bool frontier_applies(const kites_graph *g, int op, const kites_run_opts &o) {
   if (g->density_set || g->tuning || g->n + g->m / kSeg > 0xFFF00000ull) return false;
   if (o.strategy == KITES_STRATEGY_PLAIN) return true;
   return o.strategy == KITES_STRATEGY_AUTO && g->eng->sel_default && o.selector_margin < 0.f &&
-         g->coarse_strategy == KITES_STRATEGY_PULL_ALL;
+         g->coarse_strategy == KITES_STRATEGY_PULL_ALL && !g->tpv_set;
 }
 
 // Runs `op` from the start `seed` describes.  KITES_ERR_UNSUPPORTED (without
@@ -3270,6 +3270,7 @@ extern "C" int kites_graph_set_tpv(kites_graph *g, int strategy) {
     }
     g->tpv_strategy = strategy;
   }
+  if (!g->tuning) g->tpv_set = true;
   return KITES_OK;
 }
 

@@ -147,6 +147,7 @@ struct kites_graph {
   void *fr_mem = nullptr;            // k_frontier_run's buffers (allocated on first use)
   bool given = true;                 // V holds a start the caller put there, no run's result
   bool density_set = false;          // kites_graph_set_density was called
+  bool tpv_set = false;              // kites_graph_set_tpv was called
   bool tuning = false;               // kites_autotune is timing the per-iteration loops
 
   // time_kernels: one record per iteration of the last host-loop run (pull

@@ -219,6 +219,25 @@ def test_tpv_guard_on_hub_graph(engine):
         g.close()
 
 
+def test_threads_per_vertex_set_by_hand():
+    """AUTO uses the width a caller sets: the run goes by the selector."""
+    n = 1 << 12
+    s, d, w = capi.gen_rmat(12, 16 * n, seed=2)
+    R, C, E = capi.csc_from_edges(n, s, d, w)
+    auto = capi.default_opts(strategy=capi.STRATEGY_AUTO)
+    eng = capi.Engine(0)
+    try:
+        g = capi.Graph(eng, R, C, E)
+        want, one = g.sssp(7, opts=auto)
+        assert one.kernel_launches == 1
+        g.set_tpv(capi.STRATEGY_TPV4)
+        dist, st = g.sssp(7, opts=auto)
+        assert st.kernel_launches > 1
+        np.testing.assert_array_equal(dist, want)
+    finally:
+        eng.close()
+
+
 def test_autotune_knows_the_untuned_chunk_size(engine):
     """A graph whose batched runs take chunks below 128 items untuned (K = 256:
     0.5 ms with 32, 1.0 with 256) is not tuned to larger ones."""
