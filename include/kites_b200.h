@@ -175,7 +175,8 @@ typedef struct kites_run_stats {
                                        (out-edges of changed ones where a run pushes) */
   uint64_t algorithmic_bytes;       /* sum over iterations of B_t            */
   uint64_t strategy_hist[KITES_STRATEGY_COUNT];
-  uint64_t kernel_launches;         /* engine kernels launched by the call   */
+  uint64_t kernel_launches;         /* engine kernels launched by the call; device
+                                       loops: those that had work            */
   double pull_kernel_ms;            /* time_kernels: summed pull-kernel time */
   uint64_t pull_kernel_launches;
   uint64_t pull_kernel_bytes;       /* algorithmic bytes of those launches   */

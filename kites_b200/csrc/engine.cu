@@ -561,6 +561,11 @@ void launch_expand(kites_graph *g, const void *aR, const uint32_t *aC, const uin
   }
 }
 
+// Kernels of an iteration of the device loops that have work (what else its
+// graph launches sees a closed gate and leaves): activation, pull or push, end;
+// AUTO's selector pass before them.
+constexpr uint64_t kLoopKernels = 3, kAutoLoopKernels = 4;
+
 // Enqueues the end of an iteration: clears the ranges and runs the loop check.
 int launch_end(kites_graph *g, const clear_list &cl, cudaGraphConditionalHandle h,
                int has_handle, uint64_t *launches) {
@@ -771,7 +776,7 @@ int drive_loop(kites_graph *g, const kites_run_opts &o, loop_key key, Launch lau
                                  cudaMemcpyDeviceToHost, s));
   KITES_CUDA_TRY(cudaStreamSynchronize(s));
   KITES_CUDA_TRY(cudaEventElapsedTime(ms, eng->ev0, eng->ev1));
-  if (dev_loop) *launches = 4 * hctr->iterations;  // kernels that did work
+  if (dev_loop) *launches = kLoopKernels * hctr->iterations;
   *out = *hctr;
   return KITES_OK;
 }
@@ -1374,7 +1379,7 @@ int run_auto(kites_graph *g, const kites_run_opts &o, kites_run_stats *st) {
     st->algorithmic_bytes = c.iterations * 8ull * g->nwords + 12ull * c.total_active +
                             (8ull + e_bytes) * c.total_edges + 12ull * c.total_updated +
                             8ull * c.total_out_edges;
-    st->kernel_launches += dev_loop ? 6ull * c.iterations : launches;
+    st->kernel_launches += dev_loop ? kAutoLoopKernels * c.iterations : launches;
     if (o.record_iterations) {
       KITES_TRY(record_iterations(g, c, KITES_STRATEGY_AUTO, st));
       for (uint32_t i = 0; i < nrec && i < st->n_recorded; ++i)
@@ -2053,7 +2058,7 @@ int run_batch_flex(kites_graph *g, const uint32_t *sources, uint32_t *dist_out,
     KITES_CUDA_TRY(cudaStreamSynchronize(s));
     KITES_CUDA_TRY(cudaEventElapsedTime(&ms, eng->ev0, eng->ev1));
     c = *hctr;
-    launches = 6ull * c.iterations;
+    launches = kAutoLoopKernels * c.iterations;
   } else if (autosel) {
     // Host loop: select, read the class back, run it (timed per iteration).
     run_counters *hctr = (run_counters *)eng->pinned;

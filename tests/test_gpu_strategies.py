@@ -275,3 +275,30 @@ def test_autotune_times_auto_as_it_runs(engine):
         assert r.coarse_ms < 2 * total
     finally:
         eng.close()
+
+
+def test_launches_of_the_device_loops():
+    """kernel_launches of a device loop: activation, pull or push and the end
+    of every iteration, the selector's pass where it picks, and the call's own
+    initialisation (two kernels; three in a batched call)."""
+    n = 1 << 12
+    s, d, w = capi.gen_rmat(12, 16 * n, seed=2)
+    R, C, E = capi.csc_from_edges(n, s, d, w)
+    srcs = np.arange(16, dtype=np.uint32)
+    eng = capi.Engine(0)
+    try:
+        g = capi.Graph(eng, R, C, E)
+        opts = capi.default_opts
+        st = g.sssp(7, opts=opts(strategy=capi.STRATEGY_AUTO, selector_margin=0.1))[1]
+        assert st.iterations > 1 and st.kernel_launches == 4 * st.iterations
+        st = g.sssp(7, opts=opts(strategy=capi.STRATEGY_PULL_ALL))[1]
+        assert st.iterations > 1 and st.kernel_launches == 3 * st.iterations
+        st = g.sssp_batch(srcs)[1]
+        assert st.iterations > 1 and st.kernel_launches == 3 * st.iterations + 3
+        st = g.sssp_batch(srcs, opts=opts(strategy=capi.STRATEGY_AUTO, selector_margin=0.03))[1]
+        assert st.iterations > 1 and st.kernel_launches == 4 * st.iterations + 3
+        assert capi.load().kites_graph_set_density(g._h, n, n) == capi.OK
+        st = g.sssp(7)[1]
+        assert st.iterations > 1 and st.kernel_launches == 3 * st.iterations + 2
+    finally:
+        eng.close()
