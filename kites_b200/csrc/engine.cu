@@ -60,6 +60,8 @@ static_assert(sizeof(kDefaultBatchSelector) == kParams * sizeof(float),
               "selector_batch_default.inc must hold the 1628 selector parameters");
 #endif
 
+void graph_release(kites_graph *g, void *p);
+
 int dev_alloc(kites_engine *eng, void **p, size_t bytes) {
   *p = nullptr;
   // At least 16 bytes of slack past the end: the staged sweep copies whole
@@ -67,6 +69,18 @@ int dev_alloc(kites_engine *eng, void **p, size_t bytes) {
   // bytes beyond the array.
   bytes = (bytes + 16 + 255) & ~size_t(255);
   cudaError_t e = cudaMallocFromPoolAsync(p, bytes, eng->pool, eng->stream);
+  if (e == cudaErrorMemoryAllocation) {
+    // The single-launch loop's buffers (17 bytes a vertex) are the first to go:
+    // a later run allocates them again, or does without.
+    cudaGetLastError();
+    for (kites_graph *g : eng->graphs) {
+      graph_release(g, g->fr_mem);
+      g->fr_mem = nullptr;
+    }
+    cudaStreamSynchronize(eng->stream);
+    cudaMemPoolTrimTo(eng->pool, 0);
+    e = cudaMallocFromPoolAsync(p, bytes, eng->pool, eng->stream);
+  }
   if (e != cudaSuccess) {
     cudaGetLastError();
     return fail(KITES_ERR_OOM, "device pool allocation of %zu bytes failed: %s",

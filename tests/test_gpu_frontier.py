@@ -319,3 +319,33 @@ def test_engines_of_several_threads():
     for t in threads:
         t.join()
     assert not bad, bad
+
+
+def test_buffers_give_way():
+    """What the single-launch loop keeps on a graph does not take the memory of
+    a later call: a batched run whose arrays only fit in its place succeeds."""
+    import torch
+
+    n, k = 1 << 23, 16
+    ids = np.arange(n, dtype=np.uint32)
+    s, d = ids // np.uint32(4), ids          # a tree
+    srcs = np.arange(k, dtype=np.uint32)
+    got, need, fill = [], 0, None
+    for full in (False, True):
+        eng = capi.Engine(0)
+        try:
+            g = capi.Graph.from_edges(eng, n, s, d)
+            assert g.sssp(0, op=capi.OP_BFS, out=False)[1].kernel_launches == 1
+            got.append(torch.empty((n, k), dtype=torch.int32, device="cuda"))
+            if full:                         # 64 MB less than the batched run takes
+                free = torch.cuda.mem_get_info()[0]
+                fill = torch.empty(free - need + (64 << 20), dtype=torch.uint8, device="cuda")
+            before = eng.mem_usage()[2]
+            g.sssp_batch(srcs, op=capi.OP_BFS, out=got[-1])
+            need = eng.mem_usage()[2] - before
+            assert g.sssp(0, op=capi.OP_BFS, out=False)[1].iterations > 1
+        finally:
+            fill = None
+            torch.cuda.empty_cache()
+            eng.close()
+    assert torch.equal(*got)
