@@ -12,7 +12,7 @@ divided by the time.  The CSC (2.2 GB) and the 64-wide distance array
 
 The headline value runs the 64 sources as batches (V x K vertex-major
 distances, one pass per in-edge for all K sources); the same sources run
-one at a time through the plain kernel are timed alongside ("plain").
+one at a time by PLAIN kites_sssp calls are timed alongside ("plain").
 
 Multi-GPU: replicas only -- each rank runs its own sources on its own copy
 of the graph (weak scaling); torch.distributed carries only the barrier and
@@ -569,8 +569,9 @@ def run_ours(args):
                          "ms_per_step": qms / args.steps}
 
     # Rooflines of the dominant kernels, timed live with CUDA events around
-    # every launch (host loop): k_pull_batch for the headline, k_pull_chunked
-    # for the plain kernel's traversal phase.
+    # every launch (host loop): k_pull_batch for the headline, and the pulls of
+    # the per-iteration plain loop, which timed runs keep to; an untimed plain
+    # call is the single-launch loop's one kernel.
     peaks_path = os.path.join(ROOT, "MEASURED_PEAKS.json")
     peaks = json.load(open(peaks_path)) if os.path.exists(peaks_path) else {}
     peak = peaks.get("hbm_gbs", 6650.0)
@@ -734,16 +735,16 @@ def run_ours(args):
                          if b_ach is not None else
                          {"bound": "hbm", "achieved": p_ach, "peak": peak, "unit": "GB/s",
                           "frac": p_ach / peak, "traffic": None,
-                          "kernel": "k_pull_chunked + k_sweep + k_sweep_changed<SSSP> (plain pull)",
+                          "kernel": "k_pull_chunked + k_sweep + k_sweep_changed<SSSP> (plain pull of the per-iteration loop)",
                           "launches": k_launch, "peak_source": src_note}),
             "roofline_plain": {"bound": "hbm", "achieved": p_ach, "peak": peak,
                                "unit": "GB/s", "frac": p_ach / peak,
-                               "kernel": "k_pull_chunked + k_sweep + k_sweep_changed<SSSP> (plain pull phase)",
+                               "kernel": "k_pull_chunked + k_sweep + k_sweep_changed<SSSP> (plain pull phase of the per-iteration loop, which `plain` does not run)",
                                "launches": k_launch,
                                "peak_source": src_note},
             "roofline_plain_dense": ({"bound": "hbm", "achieved": d_ach, "peak": peak,
                                       "unit": "GB/s", "frac": d_ach / peak,
-                                      "kernel": "k_sweep<SSSP, row filter> + k_sweep_changed<SSSP> (dense iterations)",
+                                      "kernel": "k_sweep<SSSP, row filter> + k_sweep_changed<SSSP> (dense iterations of the per-iteration loop)",
                                       "launches": d_launch, "peak_source": src_note}
                                      if d_ach is not None else None),
             "cpu_baseline": cpu,

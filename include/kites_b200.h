@@ -168,13 +168,17 @@ typedef struct kites_run_opts {
 #define KITES_MAX_RECORDED_ITERS 4096
 
 typedef struct kites_run_stats {
-  uint64_t iterations;              /* kernel iterations, as compute.cuh:135 counts */
+  uint64_t iterations;              /* kernel iterations, as compute.cuh:135 counts; of
+                                       the single-launch loop the rounds over its
+                                       queue, which with weights are ordered by
+                                       distance and may be more */
   double device_ms;                 /* CUDA-event time of the iteration loop */
   double host_ms;                   /* wall time of the whole call           */
   uint64_t edges_traversed;         /* sum over iterations of in-edges of active vertices
                                        (out-edges of changed ones where a run pushes) */
   uint64_t algorithmic_bytes;       /* sum over iterations of B_t            */
-  uint64_t strategy_hist[KITES_STRATEGY_COUNT];
+  uint64_t strategy_hist[KITES_STRATEGY_COUNT];   /* iterations by strategy; the
+                                       single-launch loop's all as PLAIN     */
   uint64_t kernel_launches;         /* engine kernels launched by the call; device
                                        loops: those that had work            */
   double pull_kernel_ms;            /* time_kernels: summed pull-kernel time */

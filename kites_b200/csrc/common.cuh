@@ -114,17 +114,6 @@ __device__ __forceinline__ uint32_t run_mask(uint32_t owner, bool *is_head) {
   return hi & ~lo;
 }
 
-// Owner lane of virtual edge i (largest j with ex[j] <= i; a lane with no
-// edges shares its ex with the next lane, so the search lands on a lane
-// that owns edges).
-__device__ __forceinline__ uint32_t owner_of(const uint32_t *ex, uint32_t i) {
-  uint32_t j = 0;
-#pragma unroll
-  for (uint32_t step = 16; step; step >>= 1)
-    if (ex[j + step] <= i) j += step;
-  return j;
-}
-
 __device__ __forceinline__ uint32_t sat_add(uint32_t a, uint32_t b) {
   uint32_t s = a + b;
   return s < a ? kInf : s;

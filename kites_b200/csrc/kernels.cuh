@@ -67,6 +67,17 @@ struct row_slice {
   OffT *lo;
 };
 
+// Owner lane of virtual edge i (largest j with ex[j] <= i; a lane with no
+// edges shares its ex with the next lane, so the search lands on a lane
+// that owns edges).
+__device__ __forceinline__ uint32_t owner_of(const uint32_t *ex, uint32_t i) {
+  uint32_t j = 0;
+#pragma unroll
+  for (uint32_t step = 16; step; step >>= 1)
+    if (ex[j + step] <= i) j += step;
+  return j;
+}
+
 // Folds p(e) over the slice's `total` virtual edges into acc[owner] with a
 // warp-segmented min.  The policy splits each edge into a streaming load
 // (C, and E when needed) and a dependent value (the V gather), so kUnroll

@@ -22,7 +22,10 @@
 // where warps draw batches from a ticket counter and keep the next window's
 // edges loading under the current one's gathers.
 //
-// Order of work.  With weights, candidates at or above a threshold are put
+// Order of work (near and far lists as in Davidson et al., "Work-efficient
+// parallel GPU methods for single-source shortest paths", 2014; the bottom-up
+// BFS step is that of Beamer et al., "Direction-optimizing breadth-first
+// search", 2012).  With weights, candidates at or above a threshold are put
 // aside (the far list) until everything below it has settled; the threshold
 // then moves by a step that follows the work: small iterations double it (an
 // iteration costs its latency whatever it holds), large ones halve it (less
@@ -66,7 +69,7 @@ constexpr uint32_t kFlush = 128;              // queue entries a warp appends to
 constexpr uint32_t kFarFlush = 96;
 constexpr uint32_t kBatchEdges = 1024;        // out-edges of a wide batch, about
 constexpr uint64_t kFrItems = 512;            // vertices + out-edges that earn a CTA
-constexpr uint64_t kSplitEdges = 16u << 20;   // threshold rule, see run()
+constexpr uint64_t kSplitEdges = 16u << 20;   // see split_pays()
 constexpr uint32_t kWideLow = 768u << 10, kWideHigh = 4u << 20;
 
 // Counters of one step: the queues it consumes and the tickets taken from
@@ -651,6 +654,17 @@ struct frontier_run {
     }
   }
 
+  // Whether a weighted run is ordered by threshold: it relaxes less and takes
+  // more iterations for it, so it pays where there is much to relax.  Unordered
+  // -> ordered, means of 2-4 sources: Erdos-Renyi 16 edges a vertex, 2^24 edges
+  // 1.04 -> 0.72 ms, 2^26 3.56 -> 1.60; R-MAT 2^24 0.54 -> 0.53, 2^26 1.45 -> 1.41;
+  // smaller ones lose (R-MAT 2^20 0.18 -> 0.22, 2^23 0.41 -> 0.45; Erdos-Renyi 2^20
+  // 0.25 -> 0.29).  Graphs with few edges a vertex are deep, and each wave that
+  // arrives late relaxes again all that lies behind it: 2^21 vertices and 2^23
+  // edges 0.93 -> 0.68, grids of 9 M vertices 126 -> 77, 4.2 M 44 -> 36, 1.05 M
+  // 14.5 -> 13.1; the small ones among them lose a little (grid of 2^18 vertices
+  // 5.9 -> 6.3, 2^18 vertices and 2^20 edges 0.27 -> 0.35).
+  __device__ bool split_pays() const { return a.m >= kSplitEdges || a.m < 8 * a.n; }
   __device__ uint32_t step_up(uint32_t t) const { return t > kInf - delta ? kInf : t + delta; }
   // The threshold's step, from the mean iteration since its last move: an
   // iteration costs its latency up to some 10^5 edges and its edges beyond
@@ -762,7 +776,7 @@ struct frontier_run {
     // Step 0: everything in place, the single source queued.
     init();
     if (!end(fc, far_c)) return finish(false, true);
-    if (kW && a.m && (a.m >= kSplitEdges || a.m < 8 * a.n)) {
+    if (kW && a.m && split_pays()) {
       const unsigned long long mean =
           __ldcg(&a.ctl->wsum) / ((unsigned long long)gridDim.x * 32u);
       const unsigned long long d = 4ull * mean * a.n / a.m;

@@ -12,8 +12,10 @@
 // y, added there atomically and finished by k_pr_join.  R-MAT of 2^21 vertices
 // and 2^25 edges, 20 steps: 4.26 ms for the row-chunk walk this replaces (211
 // us a step with one window of 32 edges in flight a warp, 9 us for its
-// separate update), 2.71 ms here (136 us a step, 247 G gathers/s).  The error
-// against 64 bits fell from 1.1e-7 to 7e-8: longer runs are summed pairwise.
+// separate update), 2.71 ms here (136 us a step, 247 G gathers/s).  The
+// relative error against 64 bits is no larger: 8.8e-8 here and 9.5e-8 there,
+// means of four graphs of that size; single runs of either lie between 7e-8 and
+// 1.2e-7, as the order of the atomics has it.
 #pragma once
 #include "kernels_sweep.cuh"
 
