@@ -332,8 +332,6 @@ int build_out_csr(kites_graph *g, const uint32_t *row) {
   g->outR = p;
   KITES_TRY(graph_alloc(g, &p, (n + 1) * sizeof(uint32_t)));
   g->out_deg = (uint32_t *)p;
-  KITES_TRY(graph_alloc(g, &p, 16));
-  g->e_sum = (unsigned long long *)p;
   // Row ends are 32-bit edge numbers.
   if (m > 0xFFFFFFFFull)
     return fail(KITES_ERR_UNSUPPORTED, "out-CSR build supports < 2^32 edges");
@@ -374,6 +372,9 @@ void note_view(kites_graph *g) {
   if (cudaStreamIsCapturing(g->eng->stream, &cap) != cudaSuccess ||
       cap != cudaStreamCaptureStatusNone)
     return;
+  void *p;
+  if (graph_alloc(g, &p, 16) != KITES_OK) return;
+  g->e_sum = (unsigned long long *)p;
   g->e_sum_known = sum_weights(g, g->e_sum) == KITES_OK;
 }
 
@@ -383,6 +384,11 @@ int refresh_weights(kites_graph *g) {
   if (!g->viewed || g->esize != 4 || !g->m) return KITES_OK;
   kites_engine *eng = g->eng;
   cudaStream_t s = eng->stream;
+  if (!g->e_sum) {
+    void *p;
+    KITES_TRY(graph_alloc(g, &p, 16));
+    g->e_sum = (unsigned long long *)p;
+  }
   KITES_TRY(sum_weights(g, g->e_sum + 1));
   unsigned long long *h = (unsigned long long *)((char *)eng->pinned + 3072);
   KITES_CUDA_TRY(cudaMemcpyAsync(h, g->e_sum, 16, cudaMemcpyDeviceToHost, s));
