@@ -10,7 +10,6 @@
 #include <algorithm>
 #include <chrono>
 #include <type_traits>
-#include <utility>
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
 
@@ -2832,7 +2831,7 @@ extern "C" int kites_graph_set_values(kites_graph *g, const void *src, uint64_t 
   if (!g || !src) return fail(KITES_ERR_INVALID, "null argument");
   if (n > g->n) return fail(KITES_ERR_INVALID, "too many values");
   KITES_TRY(set_device(g->eng));
-  g->given = !looks_settled(g, src, n);
+  g->values = looks_settled(g, src, n) ? kValuesSettled : kValuesGiven;
   KITES_CUDA_TRY(cudaMemcpyAsync(g->V, src, n * g->vsize, cudaMemcpyDefault, g->eng->stream));
   KITES_CUDA_TRY(cudaStreamSynchronize(g->eng->stream));
   return KITES_OK;
@@ -2874,12 +2873,20 @@ extern "C" int kites_process(kites_engine *eng, kites_graph *g, int op,
   KITES_TRY(check_graph(eng, g));
   // Values that a run left are settled as a rule, and the frontier then says
   // where there is anything to do: the per-iteration loop pulls its rows alone.
-  const bool start = std::exchange(g->given, false) || g->m <= kGivenEdges;
+  const bool start = g->values == kValuesGiven ||
+                     (g->values == kValuesSettled && g->m <= kGivenEdges);
+  bool declined = false;
   if (start && (!opts || opts->strategy == KITES_STRATEGY_PLAIN) && frontier_ready(g, op, opts)) {
+    g->values = kValuesSettled;
     const int st = run_frontier(g, op, kSeedFinite, 0, stats);
     if (st != KITES_ERR_UNSUPPORTED) return st;
+    g->values = kValuesUneven;
+    declined = true;
   }
-  return run_plain_op(g, op, opts, stats);
+  const int st = run_plain_op(g, op, opts, stats);
+  if (g->values == kValuesGiven && st == KITES_OK) g->values = kValuesSettled;
+  if (st == KITES_OK && stats && declined) ++stats->kernel_launches;
+  return st;
 }
 
 // Runs `op` with a strategy other than PLAIN from the changed set already in
@@ -2923,7 +2930,7 @@ extern "C" int kites_sssp(kites_engine *eng, kites_graph *g, int op, uint32_t so
                           kites_run_stats *stats) {
   clear_error();
   KITES_TRY(check_graph(eng, g));
-  g->given = false;
+  g->values = kValuesSettled;
   if (op != OP_SSSP && op != OP_SSSP_WRAP && op != OP_BFS)
     return fail(KITES_ERR_INVALID, "kites_sssp takes SSSP, SSSP_WRAP or BFS");
   if (source >= g->n_given) return fail(KITES_ERR_INVALID, "source %u out of range", source);
@@ -2961,7 +2968,7 @@ extern "C" int kites_cc(kites_engine *eng, kites_graph *g, uint32_t *labels_out,
                         const kites_run_opts *opts, kites_run_stats *stats) {
   clear_error();
   KITES_TRY(check_graph(eng, g));
-  g->given = false;
+  g->values = kValuesSettled;
   cudaStream_t s = eng->stream;
   auto t0 = std::chrono::steady_clock::now();
   if (frontier_ready(g, OP_CC, opts)) {
@@ -2988,7 +2995,7 @@ extern "C" int kites_pagerank(kites_engine *eng, kites_graph *g, uint64_t n_real
                               kites_run_stats *stats) {
   clear_error();
   KITES_TRY(check_graph(eng, g));
-  g->given = false;
+  g->values = kValuesSettled;
   if (n_real == 0 || n_real > g->n) return fail(KITES_ERR_INVALID, "bad n_real");
   kites_run_opts o = resolve_opts(opts);
   if (stats) memset(stats, 0, sizeof(*stats));
@@ -3067,7 +3074,7 @@ extern "C" int kites_sssp_multi_seed(kites_engine *eng, kites_graph *g, int op,
                                      kites_run_stats *stats) {
   clear_error();
   KITES_TRY(check_graph(eng, g));
-  g->given = false;
+  g->values = kValuesSettled;
   if (op != OP_SSSP && op != OP_SSSP_WRAP && op != OP_BFS)
     return fail(KITES_ERR_INVALID, "multi-seed runs take SSSP, SSSP_WRAP or BFS");
   if (!seeds || n_seeds == 0) return fail(KITES_ERR_INVALID, "no seeds");
@@ -3115,7 +3122,7 @@ extern "C" int kites_selector_record(kites_engine *eng, kites_graph *g, int op, 
                                      uint32_t *n_records) {
   clear_error();
   KITES_TRY(check_graph(eng, g));
-  g->given = false;
+  g->values = kValuesSettled;
   if (!features || !times_ms || !n_records || capacity == 0)
     return fail(KITES_ERR_INVALID, "null output or zero capacity");
   if (op != OP_SSSP && op != OP_BFS && op != OP_CC)

@@ -33,6 +33,11 @@ struct kites_engine {
 
 namespace kites_internal {
 
+// What a graph's values are, as far as the calls on it tell: put there by the
+// caller; left by a run; left by a kites_process from a start that the
+// single-launch loop had declined, which it would decline again.
+enum : int { kValuesGiven, kValuesSettled, kValuesUneven };
+
 struct loop_key {
   int op;
   int strategy;
@@ -145,7 +150,7 @@ struct kites_graph {
   unsigned long long *e_sum = nullptr;
 
   void *fr_mem = nullptr;            // k_frontier_run's buffers (allocated on first use)
-  bool given = true;                 // V holds a start the caller put there, no run's result
+  int values = kites_internal::kValuesGiven;   // what V holds, for kites_process
   bool density_set = false;          // kites_graph_set_density was called
   bool tpv_set = false;              // kites_graph_set_tpv was called
   bool tuning = false;               // kites_autotune is timing the per-iteration loops

@@ -189,6 +189,33 @@ def test_process_states(engine, op, oop, state):
         g.close()
 
 
+def test_process_of_an_uneven_state(engine):
+    """A start with unsatisfied edges outside the frontier is offered to the
+    single-launch loop once, not by every call that goes on from it; values
+    set anew are."""
+    n = 3001
+    s, d, w = capi.gen_rmat(12, 20000, seed=5, n_vertices=n)
+    R, C, E = capi.csc_from_edges(n, s, d, w)
+    g = capi.Graph(engine, R, C, E)
+    try:
+        V = np.full(n, INF, np.uint32)
+        V[s[5]] = 0
+        none = np.zeros(g.n_padded // 32, np.uint32)
+        for _ in range(2):
+            g.set_values(V)
+            for call in range(3):      # nothing to do in this frontier, much outside it
+                g.set_frontier(none, n)
+                st = g.process(capi.OP_SSSP)
+                assert st.kernel_launches == 3 * st.iterations + (call == 0)
+                np.testing.assert_array_equal(g.get_values(n), V)
+        want = oracle(R, C, E, n, [int(s[5])], O.OP_SSSP_SAT)
+        np.testing.assert_array_equal(g.sssp(int(s[5]))[0], want)
+        st = g.process(capi.OP_SSSP)
+        assert st.kernel_launches == 1
+    finally:
+        g.close()
+
+
 @pytest.mark.parametrize("again", [False, True])
 def test_process_of_a_settled_state(engine, again):
     """From settled values, left by a run or set again, a small frontier costs
