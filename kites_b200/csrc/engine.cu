@@ -228,7 +228,7 @@ struct scratch {
   explicit scratch(kites_engine *e) : eng(e) {}
   scratch(const scratch &) = delete;
   ~scratch() {
-    for (void *p : held) cudaFreeAsync(p, eng->stream);
+    for (; !held.empty(); held.pop_back()) cudaFreeAsync(held.back(), eng->stream);
   }
   template <class T>
   int get(T **out, size_t bytes) {
@@ -262,12 +262,29 @@ int scan_row_ends(kites_engine *eng, const uint32_t *first, const uint32_t *last
   return KITES_OK;
 }
 
+int alloc_out_edges(kites_graph *g) {
+  void *p;
+  KITES_TRY(graph_alloc(g, &p, g->m * 4));
+  g->outC = (uint32_t *)p;
+  KITES_TRY(graph_alloc(g, &p, g->m * 4));
+  g->outE = (uint32_t *)p;
+  return KITES_OK;
+}
+
+// Above this many weighted edges the transposition keeps to the memory that a
+// sort of edge numbers would need.
+constexpr uint64_t kLeanEdges = 1ull << 30;
+
 // Sorts the edges by source, stably, and unpacks them into outC, outE and the
 // sources' row ends.  Bytes an edge at the most, with the graph's own arrays
-// (C, E, the rows): weighted 36 while the sort runs -- its keys and payload
-// twice, between which the passes go to and fro, so that CUB needs no second
-// pair of its own (12 more) and outC and outE can wait for the sort's end --,
-// unweighted 24.
+// (C, E, the rows, outC, outE): unweighted 32, weighted 52.  Weighted graphs
+// above kLeanEdges hold 36: keys and payload go to and fro between two buffers
+// each, so that CUB needs no second pair of its own (12), and outC and outE
+// wait for the sort's end (8), so that what fits in 183 GB goes on to 4.29 G
+// edges.  Both take the same time (2^24 edges and a query: 2.36 and 2.35 ms);
+// smaller graphs keep the order of allocations in which the arrays that live
+// on come first, behind which the pool placed later ones better (PageRank on
+// 2^21 vertices after other graphs: 2.71 and 2.83 ms).
 template <typename PayT>
 int transpose_edges(kites_graph *g, const uint32_t *row, uint32_t *ends) {
   kites_engine *eng = g->eng;
@@ -275,45 +292,46 @@ int transpose_edges(kites_graph *g, const uint32_t *row, uint32_t *ends) {
   const uint64_t n = g->n, m = g->m;
   const int bits = bits_for(n);
   const unsigned grid = grid_of_edges(m, kBuildPer);
+  constexpr bool kWeighted = sizeof(PayT) == 8;
+  const bool lean = kWeighted && m > kLeanEdges;
   scratch tmp(eng);
-  uint32_t *keys;
-  PayT *pay;
+  uint32_t *keys, *keys2 = nullptr;
+  PayT *pay = nullptr, *sorted;
   void *temp;
   size_t temp_bytes = 0;
-  KITES_TRY(tmp.get(&keys, m * 4));
-  KITES_TRY(tmp.get(&pay, m * sizeof(PayT)));
-  if constexpr (sizeof(PayT) == 8) {
-    uint32_t *keys2;
-    PayT *pay2;
-    KITES_TRY(tmp.get(&keys2, m * 4));
-    KITES_TRY(tmp.get(&pay2, m * sizeof(PayT)));
-    k_pack_edges<<<grid, 256, 0, s>>>(row, g->C, (const uint32_t *)g->E, m, keys, pay);
+  if constexpr (kWeighted) {
+    KITES_TRY(tmp.get(&pay, m * sizeof(PayT)));
+    if (lean) KITES_TRY(tmp.get(&keys2, m * 4));
+    k_pack_edges<<<grid, 256, 0, s>>>(row, g->C, (const uint32_t *)g->E, m, keys2, pay);
     KITES_CUDA_TRY(cudaGetLastError());
-    cub::DoubleBuffer<uint32_t> dk(keys, keys2);
-    cub::DoubleBuffer<PayT> dp(pay, pay2);
+  }
+  KITES_TRY(tmp.get(&keys, m * 4));
+  KITES_TRY(tmp.get(&sorted, m * sizeof(PayT)));
+  if (lean) {
+    cub::DoubleBuffer<uint32_t> dk(keys2, keys);
+    cub::DoubleBuffer<PayT> dp(pay, sorted);
     KITES_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, temp_bytes, dk, dp, (uint64_t)m, 0,
                                                    bits, s));
     KITES_TRY(tmp.get(&temp, temp_bytes));
     KITES_CUDA_TRY(cub::DeviceRadixSort::SortPairs(temp, temp_bytes, dk, dp, (uint64_t)m, 0, bits,
                                                    s));
+    tmp.drop(temp);
     keys = dk.Current();
-    pay = dp.Current();
+    sorted = dp.Current();
     tmp.drop(dk.Alternate());
     tmp.drop(dp.Alternate());
+    KITES_TRY(alloc_out_edges(g));
   } else {
-    KITES_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, temp_bytes, g->C, keys, row, pay,
+    const PayT *in;
+    if constexpr (kWeighted) in = pay; else in = row;
+    KITES_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, temp_bytes, g->C, keys, in, sorted,
                                                    (uint64_t)m, 0, bits, s));
     KITES_TRY(tmp.get(&temp, temp_bytes));
-    KITES_CUDA_TRY(cub::DeviceRadixSort::SortPairs(temp, temp_bytes, g->C, keys, row, pay,
+    KITES_CUDA_TRY(cub::DeviceRadixSort::SortPairs(temp, temp_bytes, g->C, keys, in, sorted,
                                                    (uint64_t)m, 0, bits, s));
   }
-  tmp.drop(temp);
-  void *p;
-  KITES_TRY(graph_alloc(g, &p, m * 4));
-  g->outC = (uint32_t *)p;
-  KITES_TRY(graph_alloc(g, &p, m * 4));
-  g->outE = (uint32_t *)p;
-  k_unpack_edges<PayT><<<grid, 256, 0, s>>>(keys, pay, m, g->outC, g->outE, ends, ends + n + 1);
+  k_unpack_edges<PayT><<<grid, 256, 0, s>>>(keys, sorted, m, g->outC, g->outE, ends,
+                                            ends + n + 1);
   KITES_CUDA_TRY(cudaGetLastError());
   return KITES_OK;
 }
@@ -329,6 +347,7 @@ int build_out_csr(kites_graph *g, const uint32_t *row) {
   void *p;
   KITES_TRY(graph_alloc(g, &p, (n + 1) * sizeof(OffT)));
   g->outR = p;
+  if (g->esize != 4 || m <= kLeanEdges) KITES_TRY(alloc_out_edges(g));
   KITES_TRY(graph_alloc(g, &p, (n + 1) * sizeof(uint32_t)));
   g->out_deg = (uint32_t *)p;
   // Row ends are 32-bit edge numbers.
@@ -342,11 +361,6 @@ int build_out_csr(kites_graph *g, const uint32_t *row) {
     KITES_TRY(transpose_edges<uint64_t>(g, row, ends));
   } else if (m) {
     KITES_TRY(transpose_edges<uint32_t>(g, row, ends));
-  } else {
-    KITES_TRY(graph_alloc(g, &p, 0));
-    g->outC = (uint32_t *)p;
-    KITES_TRY(graph_alloc(g, &p, 0));
-    g->outE = (uint32_t *)p;
   }
   return scan_row_ends<OffT>(eng, ends, ends + n + 1, n, (OffT *)g->outR, g->out_deg);
 }

@@ -145,8 +145,8 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// The transposition's keys (C) and payload (row << 32 | weight).  All arrays
-// are 16-byte aligned.
+// The transposition's payload (row << 32 | weight), and its keys (C) unless
+// keys is null.  All arrays are 16-byte aligned.
 __global__ void __launch_bounds__(256)
     k_pack_edges(const uint32_t *__restrict__ row, const uint32_t *__restrict__ C,
                  const uint32_t *__restrict__ E, uint64_t m, uint32_t *__restrict__ keys,
@@ -155,14 +155,14 @@ __global__ void __launch_bounds__(256)
   if (i0 + kBuildPer <= m) {
     const uint4 r = *reinterpret_cast<const uint4 *>(row + i0);
     const uint4 w = *reinterpret_cast<const uint4 *>(E + i0);
-    *reinterpret_cast<uint4 *>(keys + i0) = *reinterpret_cast<const uint4 *>(C + i0);
+    if (keys) *reinterpret_cast<uint4 *>(keys + i0) = *reinterpret_cast<const uint4 *>(C + i0);
     ulonglong2 *to = reinterpret_cast<ulonglong2 *>(pay + i0);
     to[0] = make_ulonglong2((uint64_t)r.x << 32 | w.x, (uint64_t)r.y << 32 | w.y);
     to[1] = make_ulonglong2((uint64_t)r.z << 32 | w.z, (uint64_t)r.w << 32 | w.w);
     return;
   }
   for (uint64_t i = i0; i < m; ++i) {
-    keys[i] = C[i];
+    if (keys) keys[i] = C[i];
     pay[i] = (uint64_t)row[i] << 32 | E[i];
   }
 }

@@ -101,21 +101,31 @@ def test_edge_lists_at_any_byte(engine, offset):
         g.close()
 
 
-@pytest.mark.parametrize("weighted,per_edge", [(True, 40), (False, 36)])
-def test_upload_memory(weighted, per_edge):
-    """What an upload holds at the most (the pool keeps what it ever held): per
-    edge, the sort by source with 32-bit edge numbers as its payload needed 40
-    bytes with weights and 36 without."""
-    n, m = 1 << 16, 1 << 24
-    rng = np.random.default_rng(1)
-    C = np.sort(rng.integers(0, n, (n, m // n), dtype=np.uint32), axis=1).reshape(-1)
-    R = np.arange(n + 1, dtype=np.uint32) * np.uint32(m // n)
-    E = rng.integers(1, 256, m, dtype=np.uint32) if weighted else None
+def test_upload_memory():
+    """What an upload of more than 2^30 weighted edges holds at the most (the
+    pool keeps what it ever held): the sort by source with 32-bit edge numbers
+    as its payload needed 40 bytes an edge."""
+    import torch
+
+    n, deg = (1 << 20) + 128, 1024
+    m = n * deg
     eng = capi.Engine(0)
     try:
-        g = capi.Graph(eng, R, C, E)
+        R = torch.arange(n + 1, dtype=torch.int32, device="cuda") * deg
+        gen = torch.Generator(device="cuda")
+        gen.manual_seed(5)
+        C = torch.randint(0, 1024, (n, deg), dtype=torch.int32, device="cuda", generator=gen)
+        C += torch.arange(deg, dtype=torch.int32, device="cuda") * 1024      # ascending
+        E = torch.randint(1, 1 << 20, (m,), dtype=torch.int32, device="cuda", generator=gen)
+        torch.cuda.synchronize()
+        g = capi.Graph(eng, R, C, E, on_device=True, n_vertices=n, n_edges=m)
         pool = eng.mem_usage()[2]
-        assert pool <= per_edge * m + (96 << 20), pool / m
-        check(g, n, R, C, E)
+        assert pool <= 40 * m + (256 << 20), pool / m
+        out = [torch.empty(n, dtype=torch.int32, device="cuda") for _ in range(2)]
+        assert g.sssp(3, out=out[0])[1].kernel_launches == 1         # over the out-edges
+        g.sssp(3, out=out[1], opts=capi.default_opts(device_loop=0))   # over the in-edges
+        assert torch.equal(*out) and int((out[0] != -1).sum()) == n
     finally:
         eng.close()
+        del R, C, E
+        torch.cuda.empty_cache()
